@@ -87,6 +87,34 @@ void Context::collect() {
     pending.clear();
 }
 
+void Context::fork(int n) {
+    if (!side_fork) HMB_CUDA(cudaEventCreateWithFlags(&side_fork, cudaEventDisableTiming));
+    HMB_CUDA(cudaEventRecord(side_fork, stream));
+    for (int i = 0; i < n; ++i) {
+        if (!side[i]) HMB_CUDA(cudaStreamCreateWithFlags(&side[i], cudaStreamNonBlocking));
+        if (!side_done[i]) HMB_CUDA(cudaEventCreateWithFlags(&side_done[i], cudaEventDisableTiming));
+        HMB_CUDA(cudaStreamWaitEvent(side[i], side_fork, 0));
+    }
+}
+
+void Context::join(int n) {
+    for (int i = 0; i < n; ++i) {
+        HMB_CUDA(cudaEventRecord(side_done[i], side[i]));
+        HMB_CUDA(cudaStreamWaitEvent(stream, side_done[i], 0));
+    }
+}
+
+void Context::release_side() {
+    for (int i = 0; i < kSideStreams; ++i) {
+        if (side[i]) cudaStreamDestroy(side[i]);
+        if (side_done[i]) cudaEventDestroy(side_done[i]);
+        side[i] = nullptr;
+        side_done[i] = nullptr;
+    }
+    if (side_fork) cudaEventDestroy(side_fork);
+    side_fork = nullptr;
+}
+
 template <typename F>
 int guarded(F&& f) {
     try {
@@ -264,6 +292,7 @@ int hm_context_destroy(hm_context ctx) {
         ctx->c.numword.reset();
         cudaStreamSynchronize(ctx->c.stream);
         hmb::release_staging(ctx->c.stream);
+        ctx->c.release_side();
         if (ctx->c.own_stream) cudaStreamDestroy(ctx->c.stream);
         delete ctx;
     });

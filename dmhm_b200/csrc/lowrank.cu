@@ -14,6 +14,11 @@
 // approximation the reference computes (its factors differ only by the
 // usual sign / rotation freedom of an SVD).
 //
+// Operations whose stacks fit a CTA's registers (up to 256 rows with 32
+// columns, 128 with 64, 96 with 96; twice the rows in FP32) run in the
+// register form of round_reg.cuh; do_round below is the general form for all
+// others.
+//
 // Every device routine is written for an arithmetic type R: double (the
 // reference's precision) or float, the low-precision form used by the early
 // iterations of a mixed-precision Schulz run (inputs and outputs stay FP64;
@@ -22,8 +27,9 @@
 #include "lowrank.h"
 
 #include <algorithm>
+#include <map>
 #include <mutex>
-#include <set>
+#include <utility>
 
 namespace hmb {
 
@@ -46,10 +52,10 @@ constexpr int kJacobiSweeps = 40;  // bounded; converges in ~6-12
 // relative truncation tolerance.
 template <typename R> struct Prec;
 template <> struct Prec<double> {
-    static constexpr double jtol = 1e-15, tiny = 1e-32, tol_floor = 0.0;
+    static constexpr double jtol = 1e-15, tiny = 1e-32, reg_tiny = 1e-32, tol_floor = 0.0;
 };
 template <> struct Prec<float> {
-    static constexpr float jtol = 1e-6f, tiny = 1e-12f;
+    static constexpr float jtol = 1e-6f, tiny = 1e-12f, reg_tiny = 1e-14f;
     static constexpr double tol_floor = kLowPrecisionTolFloor;
 };
 
@@ -61,6 +67,8 @@ __device__ __forceinline__ double r_fma(double a, double b, double c) { return f
 __device__ __forceinline__ float r_fma(float a, float b, float c) { return fmaf(a, b, c); }
 __device__ __forceinline__ double r_abs(double x) { return fabs(x); }
 __device__ __forceinline__ float r_abs(float x) { return fabsf(x); }
+__device__ __forceinline__ double r_max(double a, double b) { return fmax(a, b); }
+__device__ __forceinline__ float r_max(float a, float b) { return fmaxf(a, b); }
 __device__ __forceinline__ double r_copysign(double a, double b) { return copysign(a, b); }
 __device__ __forceinline__ float r_copysign(float a, float b) { return copysignf(a, b); }
 
@@ -79,6 +87,16 @@ __device__ __forceinline__ R warp_sum(R v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
+
+}  // namespace
+}  // namespace hmb
+
+#include "round_reg.cuh"
+
+namespace hmb {
+namespace {
+
+constexpr int kRegCols = 96;   // most columns of an op of the register form
 
 template <typename R>
 __device__ R block_sum(R v, R* red) {
@@ -401,36 +419,37 @@ struct RoundShared {
     int flag;
 };
 
+// ROUND_SET and ROUND_CONCAT: [beta U2, alpha U1], [V2, V1] exactly (SET:
+// r2 = 0), zero columns beyond, by `nw` warps.
+__device__ void copy_factors(const RoundOp& op, int warp, int nw) {
+    const int m = op.m, n = op.n, lane = threadIdx.x & 31;
+    const int r2 = op.kind == ROUND_SET ? 0 : op.r2, r = op.r1 + r2;
+    const int cap = max(r, op.rout);
+    for (int c = warp; c < cap; c += nw) {
+        double* uo = op.uo + (long long)c * m;
+        double* vo = op.vo + (long long)c * n;
+        const double* u = c < r2 ? op.u2 + (long long)c * op.ldu2 : op.u1 + (long long)(c - r2) * op.ldu1;
+        const double* v = c < r2 ? op.v2 + (long long)c * op.ldv2 : op.v1 + (long long)(c - r2) * op.ldv1;
+        const double s = c < r2 ? op.beta : op.alpha;
+        for (int i = lane; i < m; i += 32) uo[i] = c >= r ? 0.0 : s * u[i];
+        for (int i = lane; i < n; i += 32) vo[i] = c >= r ? 0.0 : v[i];
+    }
+    if (threadIdx.x == 0 && op.rank_out) *op.rank_out = r;
+}
+
 // One rounding operation, executed by the whole CTA.  `dyn` holds the core
 // and the rotations in shared memory when they fit in `smem_elems` elements.
 template <typename R>
-__device__ void do_round(const RoundOp& op_in, R* dyn, long long smem_elems, RoundShared<R>& sh,
+__device__ void do_round(const RoundOp& op, R* dyn, long long smem_elems, RoundShared<R>& sh,
                          int* numflag) {
     R* red = sh.red;
     R* norms = sh.norms;
     int* order = sh.order;
-    RoundOp op = op_in;
-    if (op.r1_dev) op.r1 = min(op.r1, *op.r1_dev);
-    if (op.r2_dev) op.r2 = min(op.r2, *op.r2_dev);
     const int m = op.m, n = op.n;
     const int tid = threadIdx.x;
 
     if (op.kind == ROUND_SET || op.kind == ROUND_CONCAT) {
-        // exact: [beta U2, alpha U1], [V2, V1] (SET: r2 = 0), zero beyond
-        const int r2 = op.kind == ROUND_SET ? 0 : op.r2, r = op.r1 + r2;
-        const int cap = max(r, op.rout);
-        for_each_entry(m, cap, [&](int i, int c) {
-            op.uo[i + (long long)c * m] =
-                c >= r    ? 0.0
-                : c < r2 ? op.beta * op.u2[i + (long long)c * op.ldu2]
-                         : op.alpha * op.u1[i + (long long)(c - r2) * op.ldu1];
-        });
-        for_each_entry(n, cap, [&](int i, int c) {
-            op.vo[i + (long long)c * n] = c >= r    ? 0.0
-                                          : c < r2 ? op.v2[i + (long long)c * op.ldv2]
-                                                   : op.v1[i + (long long)(c - r2) * op.ldv1];
-        });
-        if (tid == 0 && op.rank_out) *op.rank_out = r;
+        copy_factors(op, tid >> 5, kW);
         return;
     }
 
@@ -629,6 +648,24 @@ __device__ void do_round(const RoundOp& op_in, R* dyn, long long smem_elems, Rou
     if (!dense) cta_apply_q(Vcat, n, min(n, k), n, tauV, op.vo, rout, n);
 }
 
+// An op with its addresses and its input ranks resolved.
+__device__ __forceinline__ RoundOp resolve_op(const RoundOp& src, const RelocBases& bases) {
+    RoundOp op = src;
+    op.u1 = reloc(op.u1, bases);
+    op.v1 = reloc(op.v1, bases);
+    op.u2 = reloc(op.u2, bases);
+    op.v2 = reloc(op.v2, bases);
+    op.uo = reloc(op.uo, bases);
+    op.vo = reloc(op.vo, bases);
+    op.work = reloc(op.work, bases);
+    op.rank_out = reloc(op.rank_out, bases);
+    op.r1_dev = reloc(op.r1_dev, bases);
+    op.r2_dev = reloc(op.r2_dev, bases);
+    if (op.r1_dev) op.r1 = min(op.r1, *op.r1_dev);
+    if (op.r2_dev) op.r2 = min(op.r2, *op.r2_dev);
+    return op;
+}
+
 // One CTA per worker; worker w runs ops [begin[w], begin[w+1]) in order (a
 // C block's whole operation list, each op reading the previous one's output).
 template <typename R>
@@ -642,18 +679,28 @@ round_worker_kernel(const RoundOp* __restrict__ ops, const int* __restrict__ beg
     const int w = workers[blockIdx.x];
     const int b0 = begin[w], b1 = begin[w + 1];
     for (int i = b0; i < b1; ++i) {
-        RoundOp op = ops[i];
-        op.u1 = reloc(op.u1, bases);
-        op.v1 = reloc(op.v1, bases);
-        op.u2 = reloc(op.u2, bases);
-        op.v2 = reloc(op.v2, bases);
-        op.uo = reloc(op.uo, bases);
-        op.vo = reloc(op.vo, bases);
-        op.work = reloc(op.work, bases);
-        op.rank_out = reloc(op.rank_out, bases);
-        op.r1_dev = reloc(op.r1_dev, bases);
-        op.r2_dev = reloc(op.r2_dev, bases);
-        do_round(op, dyn, smem_elems, sh, numflag);
+        do_round(resolve_op(ops[i], bases), dyn, smem_elems, sh, numflag);
+        __syncthreads();
+    }
+}
+
+// Ops whose stacks fit the register slabs (round_reg.cuh), NW warps a CTA.
+template <typename R, int NW>
+__global__ void __launch_bounds__(NW * 32, 16 / NW)
+round_reg_kernel(const RoundOp* __restrict__ ops, const int* __restrict__ begin,
+                 const int* __restrict__ workers, int cols, int rout, const RelocBases bases,
+                 int* numflag) {
+    const reground::Cta<R, NW> C{reground::Layout(NW, cols, rout), (int)(threadIdx.x >> 5),
+                                 (int)(threadIdx.x & 31)};
+    const int w = workers[blockIdx.x];
+    const int b0 = begin[w], b1 = begin[w + 1];
+    for (int i = b0; i < b1; ++i) {
+        const RoundOp op = resolve_op(ops[i], bases);
+        if (op.kind == ROUND_SET || op.kind == ROUND_CONCAT)
+            copy_factors(op, C.warp, NW);
+        else
+            reground::round_in_registers<R, NW>(op, C, R(Prec<R>::reg_tiny), Prec<R>::tol_floor,
+                                                numflag);
         __syncthreads();
     }
 }
@@ -694,26 +741,143 @@ void launch_round_ops(Context& ctx, std::vector<RoundOp>& ops, const char* name)
 
 namespace {
 
+// Once per device (contexts on several host threads may get here at once).
+template <typename K>
+void allow_smem(K kernel, size_t bytes) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    static std::mutex mu;
+    static std::map<std::pair<int, const void*>, size_t> done;
+    std::lock_guard<std::mutex> lock(mu);
+    size_t& have = done[{dev, reinterpret_cast<const void*>(kernel)}];
+    if (have >= bytes) return;
+    HMB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    have = bytes;
+}
+
+template <typename R, int NW>
+void launch_round_reg(const RoundList& L, const int* workers, const RoundList::Group& g,
+                      const RelocBases& bases, int* numflag, cudaStream_t st) {
+    const size_t bytes = (size_t)reground::Layout(NW, g.cols, g.rout).total * sizeof(R);
+    allow_smem(round_reg_kernel<R, NW>, bytes);
+    round_reg_kernel<R, NW><<<(unsigned)g.count, NW * 32, bytes, st>>>(
+        L.ops.get(), L.index.get(), workers + g.first, g.cols, g.rout, bases, numflag);
+    HMB_CHECK_LAUNCH();
+}
+
+// The groups of a list are independent (each worker writes its own block)
+// and each leaves SMs idle at its end, so they run at the same time.
 template <typename R>
 void launch_round_typed(Context& ctx, const RoundList& L, const RelocBases& bases,
                         const char* name) {
-    const long long smem = sizeof(R) == 8 ? L.smem_double : L.smem_float;
-    {
-        // once per device (contexts on several host threads may get here at once)
-        int dev = 0;
-        cudaGetDevice(&dev);
-        static std::mutex mu;
-        static std::set<int> done;
-        std::lock_guard<std::mutex> lock(mu);
-        if (done.insert(dev).second)
-            HMB_CUDA(cudaFuncSetAttribute(round_worker_kernel<R>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)(sizeof(R) == 8 ? kSmemBytes : kSmemBytesF32)));
-    }
+    int* numflag = ctx.numerical_word();
+    const RoundList::Schedule& sch = L.sched[sizeof(R) == 8 ? 0 : 1];
+    const int* workers = L.index.get() + sch.workers;
+    int parts = sch.nw_general > 0 ? 1 : 0;
+    for (const RoundList::Group& g : sch.groups) parts += g.count > 0 ? 1 : 0;
+    if (parts == 0) return;
     LaunchScope ls(ctx, name);
-    round_worker_kernel<R><<<(unsigned)L.nw, kT, smem * sizeof(R), ctx.stream>>>(
-        L.ops.get(), L.begin.get(), L.workers.get(), smem, bases, ctx.numerical_word());
-    HMB_CHECK_LAUNCH();
+    g_launches.fetch_add(parts - 1, std::memory_order_relaxed);
+    if (parts > 1) ctx.fork(parts - 1);
+    int next = 0;   // the first part stays on the context's stream
+    auto stream = [&]() { return next++ == 0 ? ctx.stream : ctx.side[next - 2]; };
+    if (sch.nw_general > 0) {
+        allow_smem(round_worker_kernel<R>, (size_t)(sizeof(R) == 8 ? kSmemBytes : kSmemBytesF32));
+        round_worker_kernel<R><<<(unsigned)sch.nw_general, kT, sch.smem * sizeof(R), stream()>>>(
+            L.ops.get(), L.index.get(), workers, sch.smem, bases, numflag);
+        HMB_CHECK_LAUNCH();
+    }
+    for (const RoundList::Group& g : sch.groups) {
+        if (g.count == 0) continue;
+        const cudaStream_t st = stream();
+        switch (g.warps) {
+            case 4: launch_round_reg<R, 4>(L, workers, g, bases, numflag, st); break;
+            default: launch_round_reg<R, 8>(L, workers, g, bases, numflag, st); break;
+        }
+    }
+    if (parts > 1) ctx.join(parts - 1);
+}
+
+}  // namespace
+
+namespace {
+
+int op_columns(const RoundOp& op) {
+    return op.kind == ROUND_DENSE ? op.n : op.r1 + (op.kind == ROUND_GENERAL ? op.r2 : 0);
+}
+
+// Warps the register form (round_reg.cuh) needs to hold an op: 4 or 8; 16 when
+// its stacks do not fit (the general kernel runs the worker then).  Small ops
+// would fit 1 or 2 warps, but every step waits for the same chain of
+// operations whatever its width, and one kernel for all ops of a list shares
+// the instruction cache (64 x 64 blocks of rank 16, whole product: 16.0 ms;
+// with 1 and 2 warps where they fit 18.8 ms, with 8 warps for all 24 ms).
+int reg_warps(const RoundOp& op, bool fp32) {
+    if (op.kind == ROUND_SET || op.kind == ROUND_CONCAT) return 4;
+    const int cols = std::max(op_columns(op), op.rout);
+    if (cols > kRegCols) return 16;
+    for (int nw = 4; nw <= 8; nw *= 2)
+        if (std::max(std::max(op.m, op.n), cols) <= reground::slab_rows(cols, nw, fp32)) return nw;
+    return 16;
+}
+
+// Relative time of an op, for the order in which workers start.
+double op_cost(const RoundOp& op) {
+    if (op.kind == ROUND_SET || op.kind == ROUND_CONCAT) return 0.1 * op.rout;
+    const double k = op_columns(op);
+    return k * (double)(op.m + op.n + 64);
+}
+
+// Appends one precision's worker list to `index`: by the kernel that runs
+// them, in the given order.
+void schedule(const std::vector<RoundOp>& ops, const std::vector<int>& begin,
+              const std::vector<int>& order, bool fp32, std::vector<int>& index,
+              RoundList::Schedule& out) {
+    const int nw = (int)begin.size() - 1;
+    std::vector<int> group(nw, 4);
+    for (int w = 0; w < nw; ++w)
+        for (int i = begin[w]; i < begin[w + 1]; ++i)
+            group[w] = std::max(group[w], reg_warps(ops[i], fp32));
+    out.workers = (int)index.size();
+    const int base = out.workers;
+    auto take = [&](auto pick) {
+        for (int w : order)
+            if (pick(group[w])) index.push_back(w);
+    };
+    take([](int need) { return need > 8; });
+    out.nw_general = (int)index.size() - base;
+    // General kernel: the core and the rotations of an op live in shared
+    // memory when they fit the launch's size, otherwise in the (L1-cached)
+    // global work area; the size is the largest need of its non-dense ops
+    // (dense compressions with larger cores take the global path), so that
+    // more CTAs share an SM.
+    long long need_max = 0;
+    for (int i = 0; i < out.nw_general; ++i)
+        for (int o = begin[index[base + i]]; o < begin[index[base + i] + 1]; ++o) {
+            const RoundOp& op = ops[o];
+            if (op.kind == ROUND_SET || op.kind == ROUND_CONCAT) continue;
+            const bool dense = op.kind == ROUND_DENSE;
+            const long long k = op_columns(op);
+            const long long ku = op.kind == ROUND_ORTHO ? op.r1 : std::min<long long>(op.m, k);
+            const long long kv = dense ? op.n : std::min<long long>(op.n, k);
+            const long long need = ku * kv + kv * kv;
+            if (!dense || need <= 3072) need_max = std::max(need_max, need);
+        }
+    out.smem = std::min<long long>(need_max, fp32 ? kSmemBytesF32 / 4 : kSmemBytes / 8);
+    for (int g = 0; g < 2; ++g) {
+        RoundList::Group& G = out.groups[g];
+        G.warps = 8 >> g;
+        G.first = (int)index.size() - base;
+        take([&](int need) { return need == G.warps; });
+        G.count = (int)index.size() - base - G.first;
+        G.cols = G.rout = 1;
+        for (int i = G.first; i < G.first + G.count; ++i)
+            for (int o = begin[index[base + i]]; o < begin[index[base + i] + 1]; ++o) {
+                if (ops[o].kind == ROUND_SET || ops[o].kind == ROUND_CONCAT) continue;
+                G.cols = std::max(G.cols, std::max(op_columns(ops[o]), ops[o].rout));
+                G.rout = std::max(G.rout, ops[o].rout);
+            }
+    }
 }
 
 }  // namespace
@@ -722,30 +886,22 @@ void upload_round_list(Context& ctx, const std::vector<RoundOp>& ops,
                        const std::vector<int>& begin, RoundList& out) {
     out.nw = 0;
     if (ops.empty() || begin.size() < 2) return;
-    // The core and the rotations of an op live in shared memory when they
-    // fit the launch's size, otherwise in the (L1-cached) global work area;
-    // the size is the largest need of the non-dense ops (dense compressions
-    // with larger cores take the global path), so that more CTAs share an SM.
-    long long need_max = 0;
-    for (const RoundOp& op : ops) {
-        if (op.kind == ROUND_SET || op.kind == ROUND_CONCAT) continue;
-        const bool dense = op.kind == ROUND_DENSE;
-        const long long k = dense ? op.n : op.r1 + (op.kind == ROUND_GENERAL ? op.r2 : 0);
-        HMB_REQUIRE(k <= kMaxK, HM_ERR_UNSUPPORTED,
-                    "low-rank rounding of more than 128 stacked columns");
-        const long long ku = op.kind == ROUND_ORTHO ? op.r1 : std::min<long long>(op.m, k);
-        const long long kv = dense ? op.n : std::min<long long>(op.n, k);
-        const long long need = ku * kv + kv * kv;
-        if (!dense || need <= 3072) need_max = std::max(need_max, need);
-    }
-    out.smem_double = std::min<long long>(need_max, kSmemBytes / 8);
-    out.smem_float = std::min<long long>(need_max, kSmemBytesF32 / 4);
+    for (const RoundOp& op : ops)
+        HMB_REQUIRE(op.kind == ROUND_SET || op.kind == ROUND_CONCAT || op_columns(op) <= kMaxK,
+                    HM_ERR_UNSUPPORTED, "low-rank rounding of more than 128 stacked columns");
     out.nw = (int)begin.size() - 1;
-    std::vector<int> workers(out.nw);
-    for (int w = 0; w < out.nw; ++w) workers[w] = w;
     out.ops.upload(ops, ctx.stream);
-    out.begin.upload(begin, ctx.stream);
-    out.workers.upload(workers, ctx.stream);
+    // the longest operation lists first, so that the last CTAs to start are
+    // short ones
+    std::vector<double> cost(out.nw, 0.0);
+    std::vector<int> order(out.nw), index(begin);
+    for (int w = 0; w < out.nw; ++w) {
+        order[w] = w;
+        for (int i = begin[w]; i < begin[w + 1]; ++i) cost[w] += op_cost(ops[i]);
+    }
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cost[a] > cost[b]; });
+    for (int fp32 = 0; fp32 < 2; ++fp32) schedule(ops, begin, order, fp32 != 0, index, out.sched[fp32]);
+    out.index.upload(index, ctx.stream);
 }
 
 void launch_round_list(Context& ctx, const RoundList& L, const RelocBases& bases,

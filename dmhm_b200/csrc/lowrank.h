@@ -46,9 +46,20 @@ struct RoundOp {
 // launch_round_workers).
 struct RoundList {
     DeviceBuffer<RoundOp> ops;
-    DeviceBuffer<int> begin, workers;
+    DeviceBuffer<int> index;   // begin (nw + 1), then the worker lists of sched
     int nw = 0;
-    long long smem_double = 0, smem_float = 0;   // shared elements per CTA
+    // Which kernel runs which worker, for the FP64 roundings and for the
+    // FP32 ones: the list at index + `workers` has first those of the general
+    // kernel, then those of the register form by warps per CTA.
+    struct Group {
+        int warps = 0, first = 0, count = 0, cols = 1, rout = 1;
+    };
+    struct Schedule {
+        int workers = 0;
+        int nw_general = 0;
+        long long smem = 0;   // shared elements per CTA of the general kernel
+        Group groups[2];
+    } sched[2];
 };
 void upload_round_list(Context& ctx, const std::vector<RoundOp>& ops,
                        const std::vector<int>& begin, RoundList& out);

@@ -77,3 +77,43 @@ def test_set_to_identity_and_conjugate():
     ref = B.Multiply(1.0, P)
     B.Conjugate()                                  # real: nothing changes
     assert np.array_equal(B.Multiply(1.0, P), ref)
+
+
+# Stacks of k = 2 rank columns on blocks of m rows (grids that halve evenly, as
+# SetToRandom needs), around the edges of the rounding kernels: fewer rows than
+# columns, slabs of 8 to 32 rows, one, two and three columns a lane (32 | 34,
+# 64 | 66), 4 and 8 warps (121 | 144 rows), past the register form (256 | 289
+# rows, 96 | 98 columns) and a tree with blocks on two levels.
+EDGES = [((12, 12), 3, 3), ((20, 20), 3, 16), ((32, 32), 3, 16), ((32, 32), 3, 17),
+         ((44, 44), 3, 15), ((48, 48), 3, 8), ((64, 64), 3, 8), ((68, 68), 3, 8),
+         ((36, 36), 3, 32), ((36, 36), 3, 33), ((40, 40), 3, 48), ((40, 40), 3, 49),
+         ((32, 32), 4, 6)]
+
+
+@pytest.mark.parametrize("sizes,L,r", EDGES)
+def test_update_with_at_kernel_edges(sizes, L, r):
+    """Each block against the best rank-r approximation by LAPACK's SVD:
+    Gaussian factors leave a relative gap above 1e-5 at the cut, so an error of
+    a few roundings (1e-15 times the factors' condition, below 1e3) stays under
+    1e-9 of the result."""
+    from oracle import dmhm_oracle as O
+    c = D.Context(0)
+    coef = D.operators.uniform_coefficients(sizes, 1)
+    S = D.operators.stencil(sizes, coef, L)
+    A = D.HMat2d(S, L, r, True, *sizes, ctx=c)
+    B = D.HMat2d(S, L, r, True, *sizes, ctx=c)
+    A.SetToRandom()
+    B.SetToRandom()
+    A.UpdateWith(-0.7, B)
+    rng = O.Rng()
+    Ao, Bo = (O.build_stencil_hmat(2, sizes, L, r, coef) for _ in range(2))
+    O.set_to_random(Ao, rng)
+    O.set_to_random(Bo, rng)
+    for a, b in zip(Ao.leaves(), Bo.leaves()):
+        if a.kind == O.DENSE:
+            a.D = a.D - 0.7 * b.D
+        else:
+            U, s, Vt = np.linalg.svd(a.U @ a.V.T - 0.7 * b.U @ b.V.T, full_matrices=False)
+            a.U, a.V = U[:, :r] * s[:r], Vt[:r].T
+    P = np.random.default_rng(5).standard_normal((sizes[0] * sizes[1], 6))
+    assert relerr(A.Multiply(1.0, P), O.multiply_dense(Ao, 1.0, P)) < 1e-9
