@@ -9,7 +9,7 @@
 // input.  Each (H-matrix, root, op) has a template -- its work lists, built
 // once and kept on the device -- and a batch of jobs runs as two launches:
 //   phase 1: T_b = W_b^T X_b for every low-rank block b of every job
-//            (W = V, or U for the transpose): for few columns one warp per
+//            (W = V, or U for the transpose): for one column one warp per
 //            row segment of a block, whole blocks per CTA; otherwise one
 //            CTA per block and 32-column tile;
 //   phase 2: for every output row tile of every job, Y_tile = alpha * (sum
@@ -414,11 +414,9 @@ void launch_zero_tiles(Context& ctx, const std::vector<std::shared_ptr<JobTempla
 }
 
 // ---------------------------------------------------------------------------
-// Wide (many columns): FP64 64 x 64 output tiles on the FP64 tensor cores
-// (mma.m8n8k4.f64), 4 warps of 32 x 32 each (4 x 4 MMA blocks, 32
-// accumulators a thread); operands staged through shared memory in chunks
-// of KC inner indices by cp.async, two stages (the next chunk loads while
-// this one is multiplied).
+// TF32, many columns: 64 x 64 output tiles, 4 warps of 32 x 32 each; operands
+// staged through shared memory in chunks of KC inner indices by cp.async, two
+// stages (the next chunk loads while this one is multiplied).
 // ---------------------------------------------------------------------------
 constexpr int WT = kWideTile;   // tile rows = tile columns
 constexpr int KC = 16;          // inner chunk
@@ -426,12 +424,10 @@ constexpr int WTHREADS = 128;   // 2 x 2 warps of 32 x 32
 constexpr int SP = WT + 8;      // smem row: fragment loads hit 32 distinct banks
 
 constexpr int NSTAGE = 2;       // chunk buffers per CTA
-template <typename E>
-struct WideSmemT {
-    E a[NSTAGE][KC][SP];   // a[buf][p][i] = A(i, p)
-    E b[NSTAGE][KC][SP];   // b[buf][p][c] = B(p, c)
+struct WideSmem32 {
+    float a[NSTAGE][KC][SP];   // a[buf][p][i] = A(i, p)
+    float b[NSTAGE][KC][SP];   // b[buf][p][c] = B(p, c)
 };
-using WideSmem = WideSmemT<double>;
 
 // The copies carry no "memory" clobber: their shared-memory destinations are
 // read only after cp_async_wait (which has one) and a barrier, and without
@@ -460,11 +456,6 @@ __device__ __forceinline__ float round_tf32(double x) {
     return __uint_as_float(r);
 }
 
-__device__ __forceinline__ void cp_async8(double* dst, const double* src, bool valid) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src),
-                 "r"(valid ? 8 : 0));
-}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
@@ -473,16 +464,6 @@ __device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
                  : "+d"(d[0]), "+d"(d[1])
                  : "d"(a), "d"(b));
-}
-
-// Accumulator slot s = (mb * 4 + nb) * 2 + h of a thread holds tile element
-// (row_of(s), col_of(s)) (the m8n8k4 C fragment: row lane/4, columns
-// 2 (lane%4) + h of MMA block (mb, nb) of the warp's 32 x 32 quarter).
-__device__ __forceinline__ int acc_row(int s, int warp, int lane) {
-    return (warp & 1) * 32 + (s >> 3) * 8 + (lane >> 2);
-}
-__device__ __forceinline__ int acc_col(int s, int warp, int lane) {
-    return (warp >> 1) * 32 + ((s >> 1) & 3) * 8 + 2 * (lane & 3) + (s & 1);
 }
 
 // TF32 tiles: slot s = ((mb * 4 + nb) * 4 + e) of MMA block (mb, nb) (16 x 8)
@@ -494,7 +475,7 @@ __device__ __forceinline__ int acc_col_tf(int s, int warp, int lane) {
     return (warp >> 1) * 32 + ((s >> 2) & 3) * 8 + 2 * (lane & 3) + (s & 1);
 }
 
-__device__ __forceinline__ void wide_mma_tf(const WideSmemT<float>& sm, int buf, int warp, int lane,
+__device__ __forceinline__ void wide_mma_tf(const WideSmem32& sm, int buf, int warp, int lane,
                                             float (&acc)[32]) {
     const int g = lane >> 2, t = lane & 3;
     const int r0 = (warp & 1) * 32 + g, c0 = (warp >> 1) * 32 + g;
@@ -520,40 +501,8 @@ __device__ __forceinline__ void wide_mma_tf(const WideSmemT<float>& sm, int buf,
     }
 }
 
-// acc += A(warp rows, chunk) B(chunk, warp columns) over one staged chunk.
-__device__ __forceinline__ void wide_mma(const WideSmem& sm, int buf, int warp, int lane,
-                                         double (&acc)[32]) {
-    const int r0 = (warp & 1) * 32 + (lane >> 2), c0 = (warp >> 1) * 32 + (lane >> 2);
-#pragma unroll
-    for (int ks = 0; ks < KC / 4; ++ks) {
-        const int p = ks * 4 + (lane & 3);
-        double a[4], b[4];
-#pragma unroll
-        for (int mb = 0; mb < 4; ++mb) a[mb] = sm.a[buf][p][r0 + mb * 8];
-#pragma unroll
-        for (int nb = 0; nb < 4; ++nb) b[nb] = sm.b[buf][p][c0 + nb * 8];
-#pragma unroll
-        for (int mb = 0; mb < 4; ++mb)
-#pragma unroll
-            for (int nb = 0; nb < 4; ++nb) {
-                double (&d)[2] = *reinterpret_cast<double(*)[2]>(&acc[(mb * 4 + nb) * 2]);
-                dmma(d, a[mb], b[nb]);
-            }
-    }
-}
-
 // B chunk: B(p, c) = Bp[p + c * ldb] for p < len, c < cols (p fastest).
-__device__ __forceinline__ void load_b_chunk(WideSmem& sm, int buf, const double* Bp, int ldb,
-                                             int len, int cols, int tid) {
-#pragma unroll
-    for (int e = tid; e < KC * WT; e += WTHREADS) {
-        const int p = e % KC, c = e / KC;
-        const bool v = p < len && c < cols;
-        cp_async8(&sm.b[buf][p][c], v ? Bp + p + (long long)c * ldb : Bp, v);
-    }
-}
-
-__device__ __forceinline__ void load_b_chunk(WideSmemT<float>& sm, int buf, const float* Bp, int ldb,
+__device__ __forceinline__ void load_b_chunk(WideSmem32& sm, int buf, const float* Bp, int ldb,
                                              int len, int cols, int tid) {
 #pragma unroll
     for (int e = tid; e < KC * WT; e += WTHREADS) {
@@ -580,16 +529,13 @@ __device__ __forceinline__ int tiles_of(const JobExec& J) { return PHASE == 1 ? 
 template <int PHASE>
 __device__ __forceinline__ const int* chunk_prefix(const JobExec& J) { return PHASE == 1 ? J.w1cp : J.tcp; }
 
-// TF: the TF32 form (FP32 copy of the blocks and of the input, TF32
-// tensor-core MMA, FP32 accumulation, FP64 output).
-// At most 128 registers a thread, so that 4 CTAs share an SM (152 without
-// the bound: 3 CTAs per SM, 2 % slower on the 128 x 128, 64-column product).
-template <int PHASE, bool TF>
+// The TF32 form: FP32 copy of the blocks and of the input, TF32 tensor-core
+// MMA, FP32 accumulation, FP64 output.
+template <int PHASE>
 __global__ void __launch_bounds__(WTHREADS, 4)
-wide_kernel(const JobExec* __restrict__ jobs, int njobs, const JobExec job0, long long C, int G) {
-    using E = typename std::conditional<TF, float, double>::type;
+wide_tf32_kernel(const JobExec* __restrict__ jobs, int njobs, const JobExec job0, long long C, int G) {
     extern __shared__ __align__(16) unsigned char wide_smem[];
-    WideSmemT<E>& sm = *reinterpret_cast<WideSmemT<E>*>(wide_smem);
+    WideSmem32& sm = *reinterpret_cast<WideSmem32*>(wide_smem);
     __shared__ int last_flag;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int b = blockIdx.x, y = blockIdx.y;
@@ -641,60 +587,40 @@ wide_kernel(const JobExec* __restrict__ jobs, int njobs, const JobExec job0, lon
                 const int p = e % KC, i = e / KC;   // W columns are contiguous
                 const bool v = p < len && i < rows;
                 const long long wo = t->wcol[v ? i : 0];
-                if constexpr (TF) {
-                    const float* w0 = J.hb32 + wo;
-                    cp_async4(&sm.a[buf][p][i], v ? w0 + c.pos + p : w0, v);
-                } else {
-                    const double* w0 = J.hb + wo;
-                    cp_async8(&sm.a[buf][p][i], v ? w0 + c.pos + p : w0, v);
-                }
+                const float* w0 = J.hb32 + wo;
+                cp_async4(&sm.a[buf][p][i], v ? w0 + c.pos + p : w0, v);
             }
-            if constexpr (TF)
-                load_b_chunk(sm, buf, J.in32 + t->in_off + c.pos + (long long)y * WT * J.ldin32,
-                             J.ldin32, len, cols, tid);
-            else
-                load_b_chunk(sm, buf, J.in + t->in_off + c.pos + (long long)y * WT * J.ldin,
-                             J.ldin, len, cols, tid);
+            load_b_chunk(sm, buf, J.in32 + t->in_off + c.pos + (long long)y * WT * J.ldin32,
+                         J.ldin32, len, cols, tid);
             c.pos += len;
             last = c.pos >= t->nin;
         } else {
             const P2T it = J.p2[c.tile];
             const P2Entry e = J.ent[c.ei];
             const int len = min(KC, e.inner - c.pos);
-            const E* Eb;
-            if constexpr (TF) Eb = J.hb32 + e.a;
-            else Eb = J.hb + e.a;
+            const float* Eb = J.hb32 + e.a;
             if (!e.transA) {
-                const E* A = Eb + it.r0 + (long long)c.pos * e.lda;
+                const float* A = Eb + it.r0 + (long long)c.pos * e.lda;
 #pragma unroll
                 for (int x = tid; x < WT * KC; x += WTHREADS) {
                     const int i = x % WT, p = x / WT;   // rows contiguous
                     const bool v = p < len && i < it.rows;
-                    if constexpr (TF) cp_async4(&sm.a[buf][p][i], v ? A + i + (long long)p * e.lda : Eb, v);
-                    else cp_async8(&sm.a[buf][p][i], v ? A + i + (long long)p * e.lda : Eb, v);
+                    cp_async4(&sm.a[buf][p][i], v ? A + i + (long long)p * e.lda : Eb, v);
                 }
             } else {
-                const E* A = Eb + c.pos + (long long)it.r0 * e.lda;
+                const float* A = Eb + c.pos + (long long)it.r0 * e.lda;
 #pragma unroll
                 for (int x = tid; x < WT * KC; x += WTHREADS) {
                     const int p = x % KC, i = x / KC;   // inner index contiguous
                     const bool v = p < len && i < it.rows;
-                    if constexpr (TF) cp_async4(&sm.a[buf][p][i], v ? A + p + (long long)i * e.lda : Eb, v);
-                    else cp_async8(&sm.a[buf][p][i], v ? A + p + (long long)i * e.lda : Eb, v);
+                    cp_async4(&sm.a[buf][p][i], v ? A + p + (long long)i * e.lda : Eb, v);
                 }
             }
-            if constexpr (TF) {
-                const float* EB;
-                int ldb;
-                if (e.b_from_t) { EB = J.T32 + e.b_off * J.k; ldb = e.ldt; }
-                else { EB = J.in32 + e.b_off; ldb = J.ldin32; }
-                load_b_chunk(sm, buf, EB + c.pos + (long long)y * WT * ldb, ldb, len, cols, tid);
-            } else {
-                const double* EB;
-                int ldb;
-                entry_b(e, J, EB, ldb);
-                load_b_chunk(sm, buf, EB + c.pos + (long long)y * WT * ldb, ldb, len, cols, tid);
-            }
+            const float* EB;
+            int ldb;
+            if (e.b_from_t) { EB = J.T32 + e.b_off * J.k; ldb = e.ldt; }
+            else { EB = J.in32 + e.b_off; ldb = J.ldin32; }
+            load_b_chunk(sm, buf, EB + c.pos + (long long)y * WT * ldb, ldb, len, cols, tid);
             c.pos += len;
             last = false;
             if (c.pos >= e.inner) {
@@ -721,11 +647,11 @@ wide_kernel(const JobExec* __restrict__ jobs, int njobs, const JobExec job0, lon
         }
         return last;
     };
-    E acc[32];
+    float acc[32];
 #pragma unroll
     for (int q = 0; q < 32; ++q) acc[q] = 0;
-    auto arow = [&](int k) { return TF ? acc_row_tf(k, warp, lane) : acc_row(k, warp, lane); };
-    auto acol = [&](int k) { return TF ? acc_col_tf(k, warp, lane) : acc_col(k, warp, lane); };
+    auto arow = [&](int k) { return acc_row_tf(k, warp, lane); };
+    auto acol = [&](int k) { return acc_col_tf(k, warp, lane); };
     // NSTAGE-deep ring: chunk q sits in buffer q % NSTAGE and is issued
     // NSTAGE - 1 chunks ahead; one commit group per chunk slot (empty past
     // the end) keeps the wait count constant
@@ -754,8 +680,7 @@ wide_kernel(const JobExec* __restrict__ jobs, int njobs, const JobExec job0, lon
         cp_async_wait<NSTAGE - 1>();
         __syncthreads();
         const int buf = (int)(q % NSTAGE);
-        if constexpr (TF) wide_mma_tf(sm, buf, warp, lane, acc);
-        else wide_mma(sm, buf, warp, lane, acc);
+        wide_mma_tf(sm, buf, warp, lane, acc);
         __syncthreads();
         if (!lastc[buf] && q + 1 < n) continue;
         // flush the tile of this chunk
@@ -779,8 +704,7 @@ wide_kernel(const JobExec* __restrict__ jobs, int njobs, const JobExec job0, lon
         auto emit = [&](int i, int c, double v) {
             if (PHASE == 1) {
                 const long long o = wt->trel[i] * J.k + wt->tj[i] + (long long)(y * WT + c) * wt->tr[i];
-                if constexpr (TF) J.T32[o] = round_tf32(v);
-                else J.T[o] = v;
+                J.T32[o] = round_tf32(v);
             } else {
                 store_out(J, it, i, y * WT + c, v);
             }
@@ -789,25 +713,23 @@ wide_kernel(const JobExec* __restrict__ jobs, int njobs, const JobExec job0, lon
             // the thread's 32 accumulators lie in 4 tile rows: their T
             // offsets are loaded once, before the stores (which the compiler
             // must otherwise assume may change them)
-            auto rslot = [](int k) { return TF ? (((k >> 4) << 1) | ((k >> 1) & 1)) : (k >> 3); };
+            auto rslot = [](int k) { return ((k >> 4) << 1) | ((k >> 1) & 1); };
             long long rbase[4], rstep[4];
             const long long kk = J.k;
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                const int i = arow(TF ? (((q >> 1) << 4) | ((q & 1) << 1)) : q * 8);
+                const int i = arow(((q >> 1) << 4) | ((q & 1) << 1));
                 const bool ok = i < rows;
                 rbase[q] = ok ? wt->trel[i] * kk + wt->tj[i] : 0;
                 rstep[q] = ok ? (long long)wt->tr[i] : 0;
             }
-            double* Tp = J.T;
             float* T32p = J.T32;
 #pragma unroll
             for (int k = 0; k < 32; ++k) {
                 const int i = arow(k), c = acol(k);
                 if (i < rows && c < cols) {
                     const long long o = rbase[rslot(k)] + (long long)(y * WT + c) * rstep[rslot(k)];
-                    if constexpr (TF) T32p[o] = round_tf32((double)acc[k]);
-                    else Tp[o] = (double)acc[k];
+                    T32p[o] = round_tf32((double)acc[k]);
                 }
             }
         } else if (whole) {
@@ -843,6 +765,378 @@ wide_kernel(const JobExec* __restrict__ jobs, int njobs, const JobExec job0, lon
         }
 #pragma unroll
         for (int k = 0; k < 32; ++k) acc[k] = 0;
+        first_piece = false;
+    }
+}
+
+// ---------------------------------------------------------------------------
+// FP64, two columns and more: 64-row x NT-column tiles, NT = 8, 16, 32 or 64,
+// on the FP64 tensor cores (mma.m8n8k4.f64), 128 threads.
+//
+// Bound by the FP64 tensor pipe from about 40 columns on, by HBM below.  The
+// operands of a chunk (16 inner indices) reach shared memory by 16-byte
+// cp.async three chunks ahead, in the order memory has them: an operand whose
+// inner index is contiguous (W, the input, T, the transposed dense leaves) as
+// rows of 16 inner indices, their eight 16-byte units exchanged between halves
+// on odd rows; the others (U, the dense leaves) as columns of 64 rows with a
+// stride of 66.  Either way the copies and the fragment loads touch each bank
+// once, and a fragment load serves two MMAs: the inner index of the first is
+// 2t, of the second 2t + 1 (t = lane % 4), for both operands.  (Copies of 8
+// bytes into one common layout, whose bank conflicts took 30 % of the time,
+// and the work-list reads in front of every chunk held the earlier kernel to
+// 23 % and 38 % of the pipe.)  Work-list entries are fetched one chunk before
+// their use.  Row blocks and column blocks of 8 beyond a tile's rows and
+// columns are not multiplied.
+// ---------------------------------------------------------------------------
+template <int NT>
+struct Tile64 {
+    static constexpr int WN = NT == 64 ? 2 : 1, WM = 4 / WN;   // warps along columns, rows
+    static constexpr int MB = 8 / WM, NB = NT / (8 * WN);      // 8 x 8 blocks of a warp
+    static constexpr int STAGES = NT == 64 ? 3 : 4;
+    static constexpr int ASZ = KC * 66;                        // doubles of an A stage
+    static constexpr int BSZ = NT * KC;
+    static constexpr size_t smem = (size_t)STAGES * (ASZ + BSZ) * sizeof(double);
+};
+
+// Two doubles src[0], src[1] (`bytes` of them valid, zeros beyond) to the
+// shared address d; `any` is a valid address for copies of nothing.
+__device__ __forceinline__ void copy_pair(unsigned d, const double* src, int bytes, bool aligned,
+                                          const double* any) {
+    if (aligned) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(bytes ? src : any),
+                     "r"(bytes));
+    } else {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(bytes ? src : any),
+                     "r"(bytes ? 8 : 0));
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d + 8),
+                     "l"(bytes > 8 ? src + 1 : any), "r"(bytes > 8 ? 8 : 0));
+    }
+}
+__device__ __forceinline__ bool even16(const double* p, long long stride) {
+    return ((reinterpret_cast<size_t>(p) | (size_t)(stride << 3)) & 15) == 0;
+}
+
+// ONE: a single job, whose description is a kernel parameter (constant memory)
+// and not a list in global memory.
+template <int PHASE, int NT, bool ONE>
+__global__ void __launch_bounds__(WTHREADS, NT == 64 ? 4 : 5)
+wide64_kernel(const JobExec* __restrict__ jobs, int njobs, const JobExec job0, long long C, int G) {
+    using TL = Tile64<NT>;
+    constexpr int MB = TL::MB, NB = TL::NB, WM = TL::WM, WN = TL::WN, ST = TL::STAGES;
+    extern __shared__ __align__(16) unsigned char wide_smem[];
+    double* const As = reinterpret_cast<double*>(wide_smem);
+    double* const Bs = As + ST * TL::ASZ;
+    // per stage: job, tile, inner indices | layout << 8 | last chunk << 9, rows | columns << 8
+    __shared__ int4 meta[ST];
+    __shared__ int last_flag;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int wm = warp % WM, wn = warp / WM;
+    const int b = blockIdx.x, y = blockIdx.y;
+    const long long g0 = split_start(b, G, C), g1 = split_start(b + 1, G, C);
+    if (g0 >= g1) return;
+    auto job = [&](int j) -> const JobExec& {
+        if constexpr (ONE) return job0;
+        else return jobs[j];
+    };
+
+    // ---- the chunk to be loaded next: this thread's addresses --------------
+    int cj = 0, ctile, cei = 0, cpos;          // job, tile, entry, inner offset
+    int rows = 0, cols = 0, inner = 0, e1 = 0;
+    bool kmajor = true, a16 = false, b16 = false;
+    const double *pa = nullptr, *pb = nullptr, *any = nullptr;
+    long long sa = 0, sb = 0, step = KC;       // strides of the thread's copies; A's chunk step
+    long long wo[4];                           // phase 1: this thread's columns of W
+    unsigned wo16 = 0;
+    const int ku = tid & 7, kr = tid >> 3;     // unit and row of an inner-contiguous copy
+    const int mu = tid & 31, mp = tid >> 5;    // unit and column of a row-contiguous copy
+    const unsigned as0 = (unsigned)__cvta_generic_to_shared(As);
+    const unsigned bs0 = (unsigned)__cvta_generic_to_shared(Bs);
+    const unsigned dk = (unsigned)(kr * KC + 2 * (ku ^ ((kr & 1) << 2))) * 8;
+    const unsigned dm = (unsigned)(mp * 66 + 2 * mu) * 8;
+    auto fetch_entry = [&]() {                 // phase 2
+        const JobExec& J = job(cj);
+        const P2Entry e = J.ent[cei];
+        inner = e.inner;
+        kmajor = e.transA != 0;
+        const int r0 = J.p2[ctile].r0;
+        const long long lda = e.lda;
+        if (kmajor) {
+            pa = J.hb + e.a + (long long)(r0 + kr) * lda + 2 * ku;
+            sa = 16 * lda;
+            step = KC;
+            a16 = even16(J.hb + e.a, lda);
+        } else {
+            pa = J.hb + e.a + r0 + 2 * mu + mp * lda;
+            sa = 4 * lda;
+            step = KC * lda;
+            a16 = even16(J.hb + e.a, lda);     // r0 is a multiple of 64
+        }
+        int ldb;
+        entry_b(e, J, pb, ldb);
+        b16 = even16(pb, ldb);
+        pb += (long long)(y * NT + kr) * ldb + 2 * ku;
+        sb = 16LL * ldb;
+    };
+    auto fetch_tile = [&]() {
+        const JobExec& J = job(cj);
+        any = J.hb;
+        cols = min(NT, J.k - y * NT);
+        if (PHASE == 1) {
+            const W1Tile* w = J.w1 + ctile;
+            rows = w->rows;
+            inner = w->nin;
+            const double* x = J.in + w->in_off;
+            b16 = even16(x, J.ldin);
+            pb = x + (long long)(y * NT + kr) * J.ldin + 2 * ku;
+            sb = 16LL * J.ldin;
+            wo16 = 0;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                wo[q] = w->wcol[min(kr + 16 * q, rows - 1)];
+                wo16 |= (wo[q] & 1) ? 0u : 1u << q;
+                wo[q] += 2 * ku;
+            }
+        } else {
+            rows = J.p2[ctile].rows;
+            e1 = J.p2[ctile].e1;
+        }
+    };
+    {
+        cj = ONE ? 0 : find_job(jobs, njobs, g0, PHASE == 2);
+        const JobExec& J = job(cj);
+        const long long local = g0 - (PHASE == 1 ? J.p1_begin : J.p2_begin);
+        const int* cp = chunk_prefix<PHASE>(J);
+        int lo = 0, hi = tiles_of<PHASE>(J) - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (cp[mid] <= local) lo = mid;
+            else hi = mid - 1;
+        }
+        while (cp[lo + 1] <= local) ++lo;      // tiles without chunks
+        ctile = lo;
+        const int kin = (int)(local - cp[lo]);
+        if (PHASE == 1) {
+            cpos = kin * KC;
+        } else {
+            int e = J.p2[lo].e0, eh = J.p2[lo].e1 - 1;
+            while (e < eh) {
+                const int mid = (e + eh + 1) >> 1;
+                if (J.ekc[mid] <= kin) e = mid;
+                else eh = mid - 1;
+            }
+            cei = e;
+            cpos = (kin - J.ekc[e]) * KC;
+        }
+        fetch_tile();
+        if (PHASE == 2) {
+            fetch_entry();
+            pa += (cpos / KC) * step;
+        }
+        pb += cpos;
+    }
+    // copies the current chunk to stage `buf` and moves on
+    auto load = [&](int buf) {
+        const int len = min(KC, inner - cpos);
+        const unsigned A = as0 + (unsigned)buf * (TL::ASZ * 8), B = bs0 + (unsigned)buf * (TL::BSZ * 8);
+        const int kbytes = max(0, min(16, (len - 2 * ku) * 8));
+        if (PHASE == 1) {
+            const double* w = any + cpos;
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                copy_pair(A + dk + q * (16 * KC * 8), w + wo[q], kr + 16 * q < rows ? kbytes : 0,
+                          (wo16 >> q) & 1, any);
+        } else {
+            const int bytes = kmajor ? kbytes : max(0, min(16, (rows - 2 * mu) * 8));
+            const int lim = kmajor ? (rows - kr + 15) >> 4 : (len - mp + 3) >> 2;
+            const unsigned d = A + (kmajor ? dk : dm), ds = kmajor ? 16 * KC * 8 : 4 * 66 * 8;
+            const double* src = pa;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                copy_pair(d + q * ds, src, q < lim ? bytes : 0, a16, any);
+                src += sa;
+            }
+        }
+        if (NT >= 16 || kr < NT) {
+            const double* src = pb;
+#pragma unroll
+            for (int q = 0; q < (NT + 15) / 16; ++q) {
+                copy_pair(B + dk + q * (16 * KC * 8), src, kr + 16 * q < cols ? kbytes : 0, b16, any);
+                src += sb;
+            }
+        }
+        cp_async_commit();
+        const int tile0 = ctile, jb = cj, rows0 = rows, cols0 = cols;
+        const bool kmaj = PHASE == 1 || kmajor;
+        bool last = false;
+        cpos += len;
+        pb += KC;
+        if (PHASE == 2) pa += step;
+        if (cpos >= inner) {
+            cpos = 0;
+            last = PHASE == 1 || ++cei >= e1;
+            if (last) {   // the next tile with chunks (possibly of the next job)
+                for (;;) {
+                    ++ctile;
+                    if (ctile >= tiles_of<PHASE>(job(cj))) {
+                        if (ONE || cj + 1 >= njobs) break;
+                        ++cj;
+                        ctile = -1;
+                        continue;
+                    }
+                    const int* cp = chunk_prefix<PHASE>(job(cj));
+                    if (cp[ctile + 1] > cp[ctile]) break;
+                }
+                if (ctile < tiles_of<PHASE>(job(cj))) {
+                    if (PHASE == 2) cei = job(cj).p2[ctile].e0;
+                    fetch_tile();
+                    if (PHASE == 2) fetch_entry();
+                }
+            } else {
+                fetch_entry();
+            }
+        }
+        if (tid == 0)
+            meta[buf] = make_int4(jb, tile0, len | (kmaj ? 256 : 0) | (last ? 512 : 0), rows0 | cols0 << 8);
+    };
+
+    double acc[MB][NB][2];
+#pragma unroll
+    for (int m = 0; m < MB; ++m)
+#pragma unroll
+        for (int n = 0; n < NB; ++n) acc[m][n][0] = acc[m][n][1] = 0.0;
+    const long long n = g1 - g0;
+#pragma unroll
+    for (int s = 0; s < ST - 1; ++s) {
+        if (s < n) load(s);
+        else cp_async_commit();
+    }
+    const int unit = ((g & 1) << 2) ^ t;   // this lane's swizzled unit of an even half row
+    bool first_piece = true;
+    int buf = 0;
+    for (long long q = 0; q < n; ++q) {
+        cp_async_wait<ST - 2>();
+        __syncthreads();
+        // every warp is done with the stage before: refill it
+        if (q + ST - 1 < n) load(buf == 0 ? ST - 1 : buf - 1);
+        else cp_async_commit();
+        const int4 mt = meta[buf];
+        const int len = mt.z & 255;
+        const int trows = mt.w & 255, tcols = mt.w >> 8;
+        const int mcnt = (((trows + 7) >> 3) - wm + WM - 1) / WM;
+        const int ncnt = (((tcols + 7) >> 3) - wn + WN - 1) / WN;
+        const bool full = mcnt == MB && ncnt == NB;
+        const double* A = As + buf * TL::ASZ;
+        const double* B = Bs + buf * TL::BSZ;
+        buf = buf + 1 == ST ? 0 : buf + 1;
+#pragma unroll
+        for (int kp = 0; kp < KC / 8; ++kp) {
+            if (8 * kp >= len) break;
+            double2 a[MB], x[NB];
+            if (PHASE == 1 || (mt.z & 256)) {
+#pragma unroll
+                for (int m = 0; m < MB; ++m)
+                    a[m] = *reinterpret_cast<const double2*>(
+                        A + (8 * (WM * m + wm) + g) * KC + 2 * (unit ^ (4 * kp)));
+            } else {
+#pragma unroll
+                for (int m = 0; m < MB; ++m) {
+                    const double* p = A + (8 * kp + 2 * t) * 66 + 8 * (WM * m + wm) + g;
+                    a[m].x = p[0];
+                    a[m].y = p[66];
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < NB; ++c)
+                x[c] = *reinterpret_cast<const double2*>(
+                    B + (8 * (WN * c + wn) + g) * KC + 2 * (unit ^ (4 * kp)));
+            if (full) {
+#pragma unroll
+                for (int m = 0; m < MB; ++m)
+#pragma unroll
+                    for (int c = 0; c < NB; ++c) dmma(acc[m][c], a[m].x, x[c].x);
+#pragma unroll
+                for (int m = 0; m < MB; ++m)
+#pragma unroll
+                    for (int c = 0; c < NB; ++c) dmma(acc[m][c], a[m].y, x[c].y);
+            } else {
+#pragma unroll
+                for (int m = 0; m < MB; ++m) {
+                    if (m >= mcnt) break;
+#pragma unroll
+                    for (int c = 0; c < NB; ++c) {
+                        if (c >= ncnt) break;
+                        dmma(acc[m][c], a[m].x, x[c].x);
+                        dmma(acc[m][c], a[m].y, x[c].y);
+                    }
+                }
+            }
+        }
+        if (!(mt.z & 512) && q + 1 < n) continue;
+        // ---- the tile (or this CTA's piece of it) is complete -------------
+        const JobExec& J = job(mt.x);
+        const long long base = PHASE == 1 ? J.p1_begin : J.p2_begin;
+        const int* cp = chunk_prefix<PHASE>(J);
+        const long long T0 = base + cp[mt.y], T1 = base + cp[mt.y + 1];
+        const bool whole = T0 >= g0 && T1 <= g1;
+        const W1Tile* wt = PHASE == 1 ? J.w1 + mt.y : nullptr;
+        P2T it{};
+        if (PHASE == 2) it = J.p2[mt.y];
+        if (whole) {
+#pragma unroll
+            for (int m = 0; m < MB; ++m) {
+                const int i = 8 * (WM * m + wm) + g;
+                if (i >= trows) continue;
+                long long rbase = 0, rstep = 0;
+                if (PHASE == 1) {
+                    rbase = wt->trel[i] * J.k + wt->tj[i];
+                    rstep = wt->tr[i];
+                }
+#pragma unroll
+                for (int c = 0; c < NB; ++c)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const int col = 8 * (WN * c + wn) + 2 * t + h;
+                        if (col >= tcols) continue;
+                        if (PHASE == 1) J.T[rbase + (long long)(y * NT + col) * rstep] = acc[m][c][h];
+                        else store_out(J, it, i, y * NT + col, acc[m][c][h]);
+                    }
+            }
+        } else {
+            double* part = J.part + ((long long)y * 2 * G) * (WT * NT);
+            double* mine = part + (2LL * b + (first_piece ? 0 : 1)) * (WT * NT);
+#pragma unroll
+            for (int m = 0; m < MB; ++m)
+#pragma unroll
+                for (int c = 0; c < NB; ++c)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+                        mine[8 * (WM * m + wm) + g + WT * (8 * (WN * c + wn) + 2 * t + h)] = acc[m][c][h];
+            __threadfence();
+            __syncthreads();
+            const long long wa = split_owner(T0, G, C), wb = split_owner(T1 - 1, G, C);
+            int* cnt = (PHASE == 1 ? J.cnt1 : J.cnt2) + (long long)mt.y * gridDim.y + y;
+            if (tid == 0) last_flag = atomicAdd(cnt, 1) == (int)(wb - wa);
+            __syncthreads();
+            if (last_flag) {
+                __threadfence();
+                const bool wa_here = split_start(wa, G, C) == T0;
+                for (int o = tid; o < WT * tcols; o += WTHREADS) {
+                    const int i = o % WT, col = o / WT;
+                    if (i >= trows) continue;
+                    double v = 0.0;
+                    for (long long w = wa; w <= wb; ++w)
+                        v += __ldcg(part + piece_slot(w, wa, wa_here) * (WT * NT) + i + WT * col);
+                    if (PHASE == 1)
+                        J.T[wt->trel[i] * J.k + wt->tj[i] + (long long)(y * NT + col) * wt->tr[i]] = v;
+                    else store_out(J, it, i, y * NT + col, v);
+                }
+                if (tid == 0) *cnt = 0;
+            }
+        }
+#pragma unroll
+        for (int m = 0; m < MB; ++m)
+#pragma unroll
+            for (int c = 0; c < NB; ++c) acc[m][c][0] = acc[m][c][1] = 0.0;
         first_piece = false;
     }
 }
@@ -1220,36 +1514,84 @@ __global__ void in_tf32_kernel(const InConv* __restrict__ cv) {
     }
 }
 
-template <bool TF>
-using WideElem = typename std::conditional<TF, float, double>::type;
-
-template <bool TF>
-void wide_grids(Context& ctx, long long c1, long long c2, int& G1, int& G2) {
-    constexpr size_t smem = sizeof(WideSmemT<WideElem<TF>>);
+// Grids and launches of the FP64 tiles (NT columns a tile).
+template <int PHASE, int NT, bool ONE>
+int wide64_grid(Context& ctx, long long chunks) {
     static std::once_flag attr_once;
     std::call_once(attr_once, [] {
-        cudaFuncSetAttribute(wide_kernel<1, TF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        cudaFuncSetAttribute(wide_kernel<2, TF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(wide64_kernel<PHASE, NT, ONE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)Tile64<NT>::smem);
     });
-    G1 = (int)std::min<long long>(c1, persistent_grid_n(ctx, wide_kernel<1, TF>, WTHREADS, smem));
-    G2 = (int)std::min<long long>(c2, persistent_grid_n(ctx, wide_kernel<2, TF>, WTHREADS, smem));
+    return (int)std::min<long long>(
+        chunks, persistent_grid_n(ctx, wide64_kernel<PHASE, NT, ONE>, WTHREADS, Tile64<NT>::smem));
 }
 
-template <bool TF>
-void launch_wide(Context& ctx, const JobExec* jobs_d, int nj, const JobExec& job0, long long n1,
-                 long long n2, int G1, int G2, int ct) {
-    constexpr size_t smem = sizeof(WideSmemT<WideElem<TF>>);
+// f(integral_constant<NT>) for nt = 8, 16, 32 or 64.
+template <typename F>
+void with_tile_columns(int nt, F f) {
+    switch (nt) {
+        case 8: f(std::integral_constant<int, 8>{}); break;
+        case 16: f(std::integral_constant<int, 16>{}); break;
+        case 32: f(std::integral_constant<int, 32>{}); break;
+        default: f(std::integral_constant<int, 64>{}); break;
+    }
+}
+
+void wide64_grids(Context& ctx, int nt, bool one, long long c1, long long c2, int& G1, int& G2) {
+    with_tile_columns(nt, [&](auto n) {
+        constexpr int NT = decltype(n)::value;
+        G1 = one ? wide64_grid<1, NT, true>(ctx, c1) : wide64_grid<1, NT, false>(ctx, c1);
+        G2 = one ? wide64_grid<2, NT, true>(ctx, c2) : wide64_grid<2, NT, false>(ctx, c2);
+    });
+}
+
+void launch_wide64(Context& ctx, int nt, const JobExec* jobs_d, int nj, const JobExec& job0, long long n1,
+                   long long n2, int G1, int G2, int ct) {
+    with_tile_columns(nt, [&](auto n) {
+        constexpr int NT = decltype(n)::value;
+        constexpr size_t smem = Tile64<NT>::smem;
+        if (n1 > 0 && G1 > 0) {
+            LaunchScope ls(ctx, "hmm_lowrank_inner");
+            const dim3 grid((unsigned)G1, (unsigned)ct);
+            if (jobs_d) wide64_kernel<1, NT, false><<<grid, WTHREADS, smem, ctx.stream>>>(jobs_d, nj, job0, n1, G1);
+            else wide64_kernel<1, NT, true><<<grid, WTHREADS, smem, ctx.stream>>>(nullptr, 1, job0, n1, G1);
+            HMB_CHECK_LAUNCH();
+        }
+        if (n2 > 0 && G2 > 0) {
+            LaunchScope ls(ctx, "hmm_row_tiles");
+            const dim3 grid((unsigned)G2, (unsigned)ct);
+            if (jobs_d) wide64_kernel<2, NT, false><<<grid, WTHREADS, smem, ctx.stream>>>(jobs_d, nj, job0, n2, G2);
+            else wide64_kernel<2, NT, true><<<grid, WTHREADS, smem, ctx.stream>>>(nullptr, 1, job0, n2, G2);
+            HMB_CHECK_LAUNCH();
+        }
+    });
+}
+
+void wide_tf32_grids(Context& ctx, long long c1, long long c2, int& G1, int& G2) {
+    constexpr size_t smem = sizeof(WideSmem32);
+    static std::once_flag attr_once;
+    std::call_once(attr_once, [] {
+        cudaFuncSetAttribute(wide_tf32_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(wide_tf32_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    });
+    G1 = (int)std::min<long long>(c1, persistent_grid_n(ctx, wide_tf32_kernel<1>, WTHREADS, smem));
+    G2 = (int)std::min<long long>(c2, persistent_grid_n(ctx, wide_tf32_kernel<2>, WTHREADS, smem));
+}
+
+void launch_wide_tf32(Context& ctx, const JobExec* jobs_d, int nj, const JobExec& job0, long long n1,
+                      long long n2, int G1, int G2, int ct) {
+    constexpr size_t smem = sizeof(WideSmem32);
     cudaStream_t st = ctx.stream;
     if (n1 > 0 && G1 > 0) {
-        LaunchScope ls(ctx, TF ? "hmm_lowrank_inner_tf32" : "hmm_lowrank_inner");
-        wide_kernel<1, TF><<<dim3((unsigned)G1, (unsigned)ct), WTHREADS, smem, st>>>(jobs_d, nj, job0,
-                                                                                    n1, G1);
+        LaunchScope ls(ctx, "hmm_lowrank_inner_tf32");
+        wide_tf32_kernel<1><<<dim3((unsigned)G1, (unsigned)ct), WTHREADS, smem, st>>>(jobs_d, nj, job0,
+                                                                                     n1, G1);
         HMB_CHECK_LAUNCH();
     }
     if (n2 > 0 && G2 > 0) {
-        LaunchScope ls(ctx, TF ? "hmm_row_tiles_tf32" : "hmm_row_tiles");
-        wide_kernel<2, TF><<<dim3((unsigned)G2, (unsigned)ct), WTHREADS, smem, st>>>(jobs_d, nj, job0,
-                                                                                    n2, G2);
+        LaunchScope ls(ctx, "hmm_row_tiles_tf32");
+        wide_tf32_kernel<2><<<dim3((unsigned)G2, (unsigned)ct), WTHREADS, smem, st>>>(jobs_d, nj, job0,
+                                                                                     n2, G2);
         HMB_CHECK_LAUNCH();
     }
 }
@@ -1319,7 +1661,7 @@ namespace {
 
 void run_jobs_direct(Context& ctx, const std::vector<MatJob>& jobs, bool tf32);
 
-// The jobs in passes of at most 8 columns (the streaming kernels).
+// The jobs in passes of at most 8 columns (the 8-column tiles).
 void run_jobs_split(Context& ctx, const std::vector<MatJob>& jobs, int kmax) {
     for (int c0 = 0; c0 < kmax; c0 += 8) {
         std::vector<MatJob> pass(jobs);
@@ -1334,9 +1676,8 @@ void run_jobs_split(Context& ctx, const std::vector<MatJob>& jobs, int kmax) {
 }
 
 // Wide pass (1) or 8-column passes (2) for an FP64 job list of 9 to 16
-// columns.  Which is faster depends on the operator: on the 256^2 operator
-// (maxRank 32) two streaming passes are 27 % faster at 9 columns and 7 % at
-// 12; on 32^2 the tensor-core pass is faster from 9 columns.  Timed once per
+// columns: one pass of the 16-column tiles or two of the 8-column ones.  Timed
+// once per
 // (layout, job count, column count) on copies of the jobs writing into
 // scratch with beta = 0 (one untimed and three timed runs of each).
 int fp64_split_choice(Context& ctx, const std::vector<MatJob>& jobs, int kmax) {
@@ -1422,10 +1763,15 @@ void run_jobs_direct(Context& ctx, const std::vector<MatJob>& jobs, bool tf32) {
     }
     // one vector, one job: stream the blocks (matvec.cu)
     if (!tf32 && jobs.size() == 1 && jobs[0].k == 1 && multiply_vector_streamed(ctx, jobs[0])) return;
-    // few columns: 32-row tiles, work split evenly over all resident warps;
-    // many columns: 64 x 64 tiles on the tensor cores (FP64, or TF32 when asked)
-    const bool wide = kmax > 8;
-    tf32 = tf32 && wide;
+    // one column: 32-row tiles, work split evenly over all resident warps;
+    // more: tiles of 64 rows on the tensor cores (FP64 at the narrowest tile
+    // that takes the columns; TF32 when asked, from 9 columns on).  Streaming
+    // kernels on the plain FP64 units took 148 us for 5 columns of the 117 x
+    // 101 operator (rank 12), the 8-column tiles take 98; 139 and 71 us for 4
+    // columns of the 128 x 128 one.
+    const bool wide = kmax > 1;
+    tf32 = tf32 && kmax > 8;
+    const int nt = kmax <= 8 ? 8 : kmax <= 16 ? 16 : kmax <= 32 ? 32 : 64;   // FP64 tile columns
     const int row_tile = wide ? 64 : 32;
     for (const MatJob& J : jobs) tmpl.push_back(get_template(ctx, *J.H, J.root, J.trans, row_tile));
     const int ct = ceil_div(std::max(kmax, 1), kWideTile);   // wide column tiles
@@ -1450,9 +1796,13 @@ void run_jobs_direct(Context& ctx, const std::vector<MatJob>& jobs, bool tf32) {
                 c1 += tmpl[j]->wc1;
                 c2 += tmpl[j]->wc2;
             }
-        if (tf32) wide_grids<true>(ctx, c1, c2, G1, G2);
-        else wide_grids<false>(ctx, c1, c2, G1, G2);
-        p_total = 2LL * std::max(G1, G2) * ct * kWideTile * kWideTile;
+        if (tf32) wide_tf32_grids(ctx, c1, c2, G1, G2);
+        else {
+            int live = 0;
+            for (const MatJob& J : jobs) live += J.k > 0;
+            wide64_grids(ctx, nt, live == 1, c1, c2, G1, G2);
+        }
+        p_total = 2LL * std::max(G1, G2) * ct * kWideTile * (tf32 ? kWideTile : nt);
     }
     // TF32: the blocks' FP32 copies, the inputs rounded once (inputs shared
     // by several jobs converted once), an FP32 intermediate
@@ -1566,15 +1916,13 @@ void run_jobs_direct(Context& ctx, const std::vector<MatJob>& jobs, bool tf32) {
     const int nj = (int)ex.size();
     if (!wide) {
         JobTemplate* single = nj == 1 ? tmpl[first_job].get() : nullptr;
-        if (kmax <= 1) launch_narrow<1>(ctx, jobs_d, nj, job0, n1, n2, rmax, single);
-        else if (kmax <= 4) launch_narrow<4>(ctx, jobs_d, nj, job0, n1, n2, rmax, single);
-        else launch_narrow<8>(ctx, jobs_d, nj, job0, n1, n2, rmax, single);
+        launch_narrow<1>(ctx, jobs_d, nj, job0, n1, n2, rmax, single);
         launch_zero_tiles(ctx, tmpl, jobs, jobs_d, job0);
         return;
     }
     HMB_REQUIRE(ct < 65536, HM_ERR_UNSUPPORTED, "too many columns");
-    if (tf32) launch_wide<true>(ctx, jobs_d, nj, job0, n1, n2, G1, G2, ct);
-    else launch_wide<false>(ctx, jobs_d, nj, job0, n1, n2, G1, G2, ct);
+    if (tf32) launch_wide_tf32(ctx, jobs_d, nj, job0, n1, n2, G1, G2, ct);
+    else launch_wide64(ctx, nt, jobs_d, nj, job0, n1, n2, G1, G2, ct);
     // row tiles without entries: output = beta * output
     launch_zero_tiles(ctx, tmpl, jobs, jobs_d, job0);
 }

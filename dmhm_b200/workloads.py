@@ -46,8 +46,8 @@ def _device_blocks(N, k):
 
 
 def matmul(k: int = 64, products: int = 3):
-    """Y = H X through hm_multiply_dense (FP64; k <= 8 takes the few-column
-    streaming kernels, wider blocks the FP64 tensor-core kernels)."""
+    """Y = H X through hm_multiply_dense (FP64; one vector streams the blocks,
+    more columns take the FP64 tensor-core tiles)."""
     ctx = Context(0)
     H = _operator_128(ctx)
     N = H.Height()

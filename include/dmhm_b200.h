@@ -228,7 +228,7 @@ HM_API int hm_tf32_kernel_choice(hm_matrix h, const double* B, int ldb, int nrhs
 /*
  * FP64 products of 9 to 16 columns (hm_multiply_dense and the H*H sampling
  * products) run either as one pass of the FP64 tensor-core 64 x 64 tiles (1)
- * or as passes of at most 8 columns through the streaming kernels (2); which
+ * or as passes of at most 8 columns (2); which
  * is faster depends on the operator.  hm_set_fp64_split(ctx, 0) (the
  * default) times both the first time a (layout, job count, column count)
  * occurs and keeps the faster; hm_fp64_split_choice reports (and if need be
