@@ -42,6 +42,8 @@ struct JobExec {
     const int* w1cp;     // wide: chunk prefix over the W1 tiles (n_w1 + 1)
     const int* tcp;      // wide: chunk prefix over the row tiles (n2 + 1)
     const int* ekc;      // wide: first chunk of each entry within its tile
+    const WideChunk* ch1;   // wide: chunks of phase 1 / 2
+    const WideChunk* ch2;
     double* part;        // wide: partials of tiles cut between CTAs (shared by all jobs)
     const P2T* p2;
     const P2Entry* ent;
@@ -784,15 +786,24 @@ wide_tf32_kernel(const JobExec* __restrict__ jobs, int njobs, const JobExec job0
 // 2t, of the second 2t + 1 (t = lane % 4), for both operands.  (Copies of 8
 // bytes into one common layout, whose bank conflicts took 30 % of the time,
 // and the work-list reads in front of every chunk held the earlier kernel to
-// 23 % and 38 % of the pipe.)  Work-list entries are fetched one chunk before
-// their use.  Row blocks and column blocks of 8 beyond a tile's rows and
-// columns are not multiplied.
+// 23 % and 38 % of the pipe.)  The chunks are described by a flat list, read
+// two chunks ahead: a rank-16 factor is one chunk, so every chunk brings new
+// addresses.  A warp whose rows or columns all lie beyond the tile does not
+// multiply; testing that per 8 x 8 block cost more than the blocks (128
+// columns of the 200 x 184 operator: 5 %).  Measured, 64 columns of the 128 x
+// 128 operator (rank 16): 392 -> 283 us for both phases, 16 TF/s of 37; 5
+// columns of the 117 x 101 one, transposed: 147 -> 82 us.
 // ---------------------------------------------------------------------------
 template <int NT>
 struct Tile64 {
     static constexpr int WN = NT == 64 ? 2 : 1, WM = 4 / WN;   // warps along columns, rows
     static constexpr int MB = 8 / WM, NB = NT / (8 * WN);      // 8 x 8 blocks of a warp
-    static constexpr int STAGES = NT == 64 ? 3 : 4;
+    static constexpr int STAGES = 3;
+    // CTAs an SM: fewer for the wide tiles, whose accumulators and addresses
+    // otherwise spill (64 columns: 3 CTAs 283 us, 4 CTAs 300 us, 4 stages 290
+    // us for the 128 x 128 operator; 8 columns: 6 CTAs 82 us, 5 CTAs 88 us for
+    // 5 columns of the 117 x 101 one)
+    static constexpr int CTAS = NT == 64 ? 3 : NT == 32 ? 4 : 6;
     static constexpr int ASZ = KC * 66;                        // doubles of an A stage
     static constexpr int BSZ = NT * KC;
     static constexpr size_t smem = (size_t)STAGES * (ASZ + BSZ) * sizeof(double);
@@ -819,7 +830,7 @@ __device__ __forceinline__ bool even16(const double* p, long long stride) {
 // ONE: a single job, whose description is a kernel parameter (constant memory)
 // and not a list in global memory.
 template <int PHASE, int NT, bool ONE>
-__global__ void __launch_bounds__(WTHREADS, NT == 64 ? 4 : 5)
+__global__ void __launch_bounds__(WTHREADS, Tile64<NT>::CTAS)
 wide64_kernel(const JobExec* __restrict__ jobs, int njobs, const JobExec job0, long long C, int G) {
     using TL = Tile64<NT>;
     constexpr int MB = TL::MB, NB = TL::NB, WM = TL::WM, WN = TL::WN, ST = TL::STAGES;
@@ -840,115 +851,97 @@ wide64_kernel(const JobExec* __restrict__ jobs, int njobs, const JobExec job0, l
     };
 
     // ---- the chunk to be loaded next: this thread's addresses --------------
-    int cj = 0, ctile, cei = 0, cpos;          // job, tile, entry, inner offset
-    int rows = 0, cols = 0, inner = 0, e1 = 0;
-    bool kmajor = true, a16 = false, b16 = false;
-    const double *pa = nullptr, *pb = nullptr, *any = nullptr;
-    long long sa = 0, sb = 0, step = KC;       // strides of the thread's copies; A's chunk step
-    long long wo[4];                           // phase 1: this thread's columns of W
-    unsigned wo16 = 0;
     const int ku = tid & 7, kr = tid >> 3;     // unit and row of an inner-contiguous copy
     const int mu = tid & 31, mp = tid >> 5;    // unit and column of a row-contiguous copy
     const unsigned as0 = (unsigned)__cvta_generic_to_shared(As);
     const unsigned bs0 = (unsigned)__cvta_generic_to_shared(Bs);
     const unsigned dk = (unsigned)(kr * KC + 2 * (ku ^ ((kr & 1) << 2))) * 8;
     const unsigned dm = (unsigned)(mp * 66 + 2 * mu) * 8;
-    auto fetch_entry = [&]() {                 // phase 2
-        const JobExec& J = job(cj);
-        const P2Entry e = J.ent[cei];
-        inner = e.inner;
-        kmajor = e.transA != 0;
-        const int r0 = J.p2[ctile].r0;
-        const long long lda = e.lda;
-        if (kmajor) {
-            pa = J.hb + e.a + (long long)(r0 + kr) * lda + 2 * ku;
-            sa = 16 * lda;
-            step = KC;
-            a16 = even16(J.hb + e.a, lda);
-        } else {
-            pa = J.hb + e.a + r0 + 2 * mu + mp * lda;
-            sa = 4 * lda;
-            step = KC * lda;
-            a16 = even16(J.hb + e.a, lda);     // r0 is a multiple of 64
-        }
-        int ldb;
-        entry_b(e, J, pb, ldb);
-        b16 = even16(pb, ldb);
-        pb += (long long)(y * NT + kr) * ldb + 2 * ku;
-        sb = 16LL * ldb;
+    int cj = ONE ? 0 : find_job(jobs, njobs, g0, PHASE == 2);
+    long long gn = g0, jend = 0;   // index of the chunk in `next`; end of its job
+    auto begin_of = [&](int j) { return PHASE == 1 ? job(j).p1_begin : job(j).p2_begin; };
+    if (!ONE) jend = cj + 1 < njobs ? begin_of(cj + 1) : C;
+    int nj = cj;                   // job of `next`
+    WideChunk next;                // the chunk after the one whose addresses are ready
+    auto fetch_next = [&]() {
+        if (gn >= g1) return;
+        if (!ONE)
+            while (gn >= jend) {
+                ++nj;
+                jend = nj + 1 < njobs ? begin_of(nj + 1) : C;
+            }
+        const JobExec& J = job(nj);
+        const int4* p = reinterpret_cast<const int4*>((PHASE == 1 ? J.ch1 : J.ch2) + (gn - begin_of(nj)));
+        const int4 u = __ldg(p), v = __ldg(p + 1);
+        next.a = (long long)(((unsigned long long)(unsigned)u.y << 32) | (unsigned)u.x);
+        next.lda = u.z;
+        next.b = u.w;
+        next.pos = v.x;
+        next.ldt = v.y;
+        next.tile = v.z;
+        next.bits = v.w;
+        ++gn;
     };
-    auto fetch_tile = [&]() {
+    int ctile = -1, cbits = 0, cols = 0, lda = 0, ldb = 0;
+    bool a16 = false, b16 = false;
+    const double *pa = nullptr, *pb = nullptr, *any = nullptr;
+    long long wo[4];                           // phase 1: this thread's columns of W
+    unsigned wo16 = 0;
+    // the addresses of `next`, which becomes the current chunk
+    auto advance = [&]() {
+        const bool new_tile = next.tile != ctile || (!ONE && nj != cj);
+        cj = nj;
         const JobExec& J = job(cj);
         any = J.hb;
+        ctile = next.tile;
+        cbits = next.bits;
         cols = min(NT, J.k - y * NT);
         if (PHASE == 1) {
-            const W1Tile* w = J.w1 + ctile;
-            rows = w->rows;
-            inner = w->nin;
-            const double* x = J.in + w->in_off;
-            b16 = even16(x, J.ldin);
-            pb = x + (long long)(y * NT + kr) * J.ldin + 2 * ku;
-            sb = 16LL * J.ldin;
-            wo16 = 0;
+            if (new_tile) {
+                const W1Tile* w = J.w1 + ctile;
+                const int rows = cbits >> 16;
+                wo16 = 0;
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                wo[q] = w->wcol[min(kr + 16 * q, rows - 1)];
-                wo16 |= (wo[q] & 1) ? 0u : 1u << q;
-                wo[q] += 2 * ku;
+                for (int q = 0; q < 4; ++q) {
+                    wo[q] = __ldg(w->wcol + min(kr + 16 * q, rows - 1));
+                    wo16 |= (wo[q] & 1) ? 0u : 1u << q;
+                    wo[q] += 2 * ku;
+                }
             }
+            pa = J.hb + next.pos;
+            ldb = J.ldin;
+            pb = J.in + next.b + next.pos;
         } else {
-            rows = J.p2[ctile].rows;
-            e1 = J.p2[ctile].e1;
+            lda = next.lda;
+            const bool km = (cbits & 256) != 0;
+            pa = J.hb + next.a;
+            a16 = ((next.a | lda) & 1) == 0;   // the storage itself is aligned
+            pa += (long long)(km ? kr : mp) * lda + 2 * (km ? ku : mu);
+            ldb = next.ldt > 0 ? next.ldt : J.ldin;
+            pb = (next.ldt > 0 ? J.T + (long long)next.b * J.k : J.in + next.b) + next.pos;
         }
+        b16 = even16(pb, ldb);
+        pb += (long long)(y * NT + kr) * ldb + 2 * ku;
+        fetch_next();
     };
-    {
-        cj = ONE ? 0 : find_job(jobs, njobs, g0, PHASE == 2);
-        const JobExec& J = job(cj);
-        const long long local = g0 - (PHASE == 1 ? J.p1_begin : J.p2_begin);
-        const int* cp = chunk_prefix<PHASE>(J);
-        int lo = 0, hi = tiles_of<PHASE>(J) - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (cp[mid] <= local) lo = mid;
-            else hi = mid - 1;
-        }
-        while (cp[lo + 1] <= local) ++lo;      // tiles without chunks
-        ctile = lo;
-        const int kin = (int)(local - cp[lo]);
-        if (PHASE == 1) {
-            cpos = kin * KC;
-        } else {
-            int e = J.p2[lo].e0, eh = J.p2[lo].e1 - 1;
-            while (e < eh) {
-                const int mid = (e + eh + 1) >> 1;
-                if (J.ekc[mid] <= kin) e = mid;
-                else eh = mid - 1;
-            }
-            cei = e;
-            cpos = (kin - J.ekc[e]) * KC;
-        }
-        fetch_tile();
-        if (PHASE == 2) {
-            fetch_entry();
-            pa += (cpos / KC) * step;
-        }
-        pb += cpos;
-    }
+    fetch_next();
+    advance();
     // copies the current chunk to stage `buf` and moves on
     auto load = [&](int buf) {
-        const int len = min(KC, inner - cpos);
+        const int len = cbits & 255, rows = cbits >> 16;
         const unsigned A = as0 + (unsigned)buf * (TL::ASZ * 8), B = bs0 + (unsigned)buf * (TL::BSZ * 8);
         const int kbytes = max(0, min(16, (len - 2 * ku) * 8));
         if (PHASE == 1) {
-            const double* w = any + cpos;
 #pragma unroll
             for (int q = 0; q < 4; ++q)
-                copy_pair(A + dk + q * (16 * KC * 8), w + wo[q], kr + 16 * q < rows ? kbytes : 0,
+                copy_pair(A + dk + q * (16 * KC * 8), pa + wo[q], kr + 16 * q < rows ? kbytes : 0,
                           (wo16 >> q) & 1, any);
         } else {
-            const int bytes = kmajor ? kbytes : max(0, min(16, (rows - 2 * mu) * 8));
-            const int lim = kmajor ? (rows - kr + 15) >> 4 : (len - mp + 3) >> 2;
-            const unsigned d = A + (kmajor ? dk : dm), ds = kmajor ? 16 * KC * 8 : 4 * 66 * 8;
+            const bool km = (cbits & 256) != 0;
+            const int bytes = km ? kbytes : max(0, min(16, (rows - 2 * mu) * 8));
+            const int lim = km ? (rows - kr + 15) >> 4 : (len - mp + 3) >> 2;
+            const unsigned d = A + (km ? dk : dm), ds = km ? 16 * KC * 8 : 4 * 66 * 8;
+            const long long sa = (long long)lda << (km ? 4 : 2);
             const double* src = pa;
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
@@ -958,6 +951,7 @@ wide64_kernel(const JobExec* __restrict__ jobs, int njobs, const JobExec job0, l
         }
         if (NT >= 16 || kr < NT) {
             const double* src = pb;
+            const long long sb = (long long)ldb << 4;
 #pragma unroll
             for (int q = 0; q < (NT + 15) / 16; ++q) {
                 copy_pair(B + dk + q * (16 * KC * 8), src, kr + 16 * q < cols ? kbytes : 0, b16, any);
@@ -965,38 +959,8 @@ wide64_kernel(const JobExec* __restrict__ jobs, int njobs, const JobExec job0, l
             }
         }
         cp_async_commit();
-        const int tile0 = ctile, jb = cj, rows0 = rows, cols0 = cols;
-        const bool kmaj = PHASE == 1 || kmajor;
-        bool last = false;
-        cpos += len;
-        pb += KC;
-        if (PHASE == 2) pa += step;
-        if (cpos >= inner) {
-            cpos = 0;
-            last = PHASE == 1 || ++cei >= e1;
-            if (last) {   // the next tile with chunks (possibly of the next job)
-                for (;;) {
-                    ++ctile;
-                    if (ctile >= tiles_of<PHASE>(job(cj))) {
-                        if (ONE || cj + 1 >= njobs) break;
-                        ++cj;
-                        ctile = -1;
-                        continue;
-                    }
-                    const int* cp = chunk_prefix<PHASE>(job(cj));
-                    if (cp[ctile + 1] > cp[ctile]) break;
-                }
-                if (ctile < tiles_of<PHASE>(job(cj))) {
-                    if (PHASE == 2) cei = job(cj).p2[ctile].e0;
-                    fetch_tile();
-                    if (PHASE == 2) fetch_entry();
-                }
-            } else {
-                fetch_entry();
-            }
-        }
-        if (tid == 0)
-            meta[buf] = make_int4(jb, tile0, len | (kmaj ? 256 : 0) | (last ? 512 : 0), rows0 | cols0 << 8);
+        if (tid == 0) meta[buf] = make_int4(cj, ctile, cbits & 0xffff, rows | cols << 8);
+        advance();   // (past the last chunk: the same addresses again, unused)
     };
 
     double acc[MB][NB][2];
@@ -1022,15 +986,14 @@ wide64_kernel(const JobExec* __restrict__ jobs, int njobs, const JobExec job0, l
         const int4 mt = meta[buf];
         const int len = mt.z & 255;
         const int trows = mt.w & 255, tcols = mt.w >> 8;
-        const int mcnt = (((trows + 7) >> 3) - wm + WM - 1) / WM;
-        const int ncnt = (((tcols + 7) >> 3) - wn + WN - 1) / WN;
-        const bool full = mcnt == MB && ncnt == NB;
+        // a warp whose blocks all lie beyond the tile has nothing to multiply
+        const bool live = 8 * wm < trows && 8 * wn < tcols;
         const double* A = As + buf * TL::ASZ;
         const double* B = Bs + buf * TL::BSZ;
         buf = buf + 1 == ST ? 0 : buf + 1;
 #pragma unroll
         for (int kp = 0; kp < KC / 8; ++kp) {
-            if (8 * kp >= len) break;
+            if (!live || 8 * kp >= len) break;
             double2 a[MB], x[NB];
             if (PHASE == 1 || (mt.z & 256)) {
 #pragma unroll
@@ -1049,27 +1012,14 @@ wide64_kernel(const JobExec* __restrict__ jobs, int njobs, const JobExec job0, l
             for (int c = 0; c < NB; ++c)
                 x[c] = *reinterpret_cast<const double2*>(
                     B + (8 * (WN * c + wn) + g) * KC + 2 * (unit ^ (4 * kp)));
-            if (full) {
 #pragma unroll
-                for (int m = 0; m < MB; ++m)
+            for (int m = 0; m < MB; ++m)
 #pragma unroll
-                    for (int c = 0; c < NB; ++c) dmma(acc[m][c], a[m].x, x[c].x);
+                for (int c = 0; c < NB; ++c) dmma(acc[m][c], a[m].x, x[c].x);
 #pragma unroll
-                for (int m = 0; m < MB; ++m)
+            for (int m = 0; m < MB; ++m)
 #pragma unroll
-                    for (int c = 0; c < NB; ++c) dmma(acc[m][c], a[m].y, x[c].y);
-            } else {
-#pragma unroll
-                for (int m = 0; m < MB; ++m) {
-                    if (m >= mcnt) break;
-#pragma unroll
-                    for (int c = 0; c < NB; ++c) {
-                        if (c >= ncnt) break;
-                        dmma(acc[m][c], a[m].x, x[c].x);
-                        dmma(acc[m][c], a[m].y, x[c].y);
-                    }
-                }
-            }
+                for (int c = 0; c < NB; ++c) dmma(acc[m][c], a[m].y, x[c].y);
         }
         if (!(mt.z & 512) && q + 1 < n) continue;
         // ---- the tile (or this CTA's piece of it) is complete -------------
@@ -1318,10 +1268,11 @@ std::shared_ptr<JobTemplate> build_template(Context& ctx, const HMatrix& H, int 
     T->c1 = c1;
     T->c2 = c2;
     T->rmax = rmax;
-    T->p1.upload(p1, ctx.stream);
+    // (the wide kernels take the W1 tiles; tc_matmul.cu the items of the whole
+    // matrix)
+    if (row_tile <= 32 || (root == 0 && !trans)) T->p1.upload(p1, ctx.stream);
     T->p2.upload(p2, ctx.stream);
     T->ent.upload(ent, ctx.stream);
-    T->zero_tiles.upload(zero, ctx.stream);
     T->hzero = zero;
     T->nw1 = (int)w1.size();
     T->w1.upload(w1, ctx.stream);
@@ -1340,9 +1291,31 @@ std::shared_ptr<JobTemplate> build_template(Context& ctx, const HMatrix& H, int 
         }
         T->wc1 = w1cp.back();
         T->wc2 = tcp.back();
-        T->w1cp.upload(w1cp, ctx.stream);
-        T->tcp.upload(tcp, ctx.stream);
-        T->ekc.upload(ekc, ctx.stream);
+        w1cp.insert(w1cp.end(), tcp.begin(), tcp.end());
+        w1cp.insert(w1cp.end(), ekc.begin(), ekc.end());
+        T->prefix.upload(w1cp, ctx.stream);
+        std::vector<WideChunk> ch;
+        ch.reserve((size_t)(T->wc1 + T->wc2));
+        for (size_t i = 0; i < w1.size(); ++i)
+            for (int pos = 0; pos < w1[i].nin; pos += KC) {
+                const int len = std::min(KC, w1[i].nin - pos);
+                ch.push_back({0, 0, (int)w1[i].in_off, pos, 0, (int)i,
+                              len | 256 | (pos + KC >= w1[i].nin ? 512 : 0) | w1[i].rows << 16});
+            }
+        for (size_t t = 0; t < p2.size(); ++t)
+            for (int e = p2[t].e0; e < p2[t].e1; ++e) {
+                const P2Entry& E = ent[e];
+                for (int pos = 0; pos < E.inner; pos += KC) {
+                    const int len = std::min(KC, E.inner - pos);
+                    const long long a = E.a + (E.transA ? pos + (long long)p2[t].r0 * E.lda
+                                                        : p2[t].r0 + (long long)pos * E.lda);
+                    ch.push_back({a, E.lda, (int)E.b_off, pos, E.b_from_t ? E.ldt : 0, (int)t,
+                                  len | (E.transA ? 256 : 0) |
+                                      (e + 1 == p2[t].e1 && pos + KC >= E.inner ? 512 : 0) |
+                                      p2[t].rows << 16});
+                }
+            }
+        T->chunks.upload(ch, ctx.stream);
     }
     T->hp1 = std::move(p1);
     T->hp2 = std::move(p2);
@@ -1395,8 +1368,9 @@ std::shared_ptr<JobTemplate> get_template(Context& ctx, const HMatrix& H, int ro
     auto it = G.templates.find(key);
     if (it != G.templates.end()) return it->second;
     auto T = build_template(ctx, H, root, trans, row_tile);
-    HMB_REQUIRE((T->n1 == 0 || T->p1.get()) && (T->n2 == 0 || (T->p2.get() && T->ent.get())) &&
-                    (T->nz == 0 || T->zero_tiles.get()) && (T->nw1 == 0 || T->w1.get()),
+    HMB_REQUIRE((T->n1 == 0 || T->p1.get() || T->w1.get()) &&
+                    (T->n2 == 0 || (T->p2.get() && T->ent.get())) && (T->nw1 == 0 || T->w1.get()) &&
+                    (T->wc1 + T->wc2 == 0 || T->chunks.get()),
                 HM_ERR_INTERNAL, "work lists missing on the device");
     G.templates.emplace(key, T);
     return T;
@@ -1883,9 +1857,13 @@ void run_jobs_direct(Context& ctx, const std::vector<MatJob>& jobs, bool tf32) {
             e.T = tbuf.get() + t_off[j];
             e.part = tbuf.get() + t_total;
         }
-        e.w1cp = T.w1cp.get();
-        e.tcp = T.tcp.get();
-        e.ekc = T.ekc.get();
+        if (wide) {
+            e.w1cp = T.prefix.get();
+            e.tcp = e.w1cp + T.nw1 + 1;
+            e.ekc = e.tcp + T.n2 + 1;
+            e.ch1 = T.chunks.get();
+            e.ch2 = e.ch1 + T.wc1;
+        }
         e.cnt1 = cnt + c1_off[j];
         e.cnt2 = cnt + c2_off[j];
         e.alpha_scale = J.alpha_scale;

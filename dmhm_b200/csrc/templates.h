@@ -50,15 +50,28 @@ struct W1Tile {
     int tr[kWideTile];
 };
 
+// One chunk (at most 16 inner indices) of a 64-row tile of the FP64 product, in
+// the order the persistent CTAs take them: phase 1 the chunks of every W1Tile,
+// phase 2 those of every row tile's entries.
+struct WideChunk {
+    long long a;   // phase 2: storage offset of A's first element of the chunk
+    int lda;
+    int b;         // first row of B: of the job input, or (ldt > 0) of T before its k-fold scale
+    int pos;       // inner offset of the chunk in B
+    int ldt;       // > 0: B is T + b k + pos with this leading dimension
+    int tile;
+    int bits;      // inner indices | inner-contiguous A << 8 | last of its tile << 9 | rows << 16
+};
+
 struct JobTemplate {
     DeviceBuffer<P1T> p1;
     DeviceBuffer<P2T> p2;
     DeviceBuffer<P2Entry> ent;
-    DeviceBuffer<int> zero_tiles;   // tiles without entries (output = beta * output)
     DeviceBuffer<W1Tile> w1;        // wide phase-1 tiles
-    DeviceBuffer<int> w1cp;         // wide: chunk prefix over the W1 tiles
-    DeviceBuffer<int> tcp;          // wide: chunk prefix over the row tiles
-    DeviceBuffer<int> ekc;          // wide: first chunk of every entry within its tile
+    // wide: chunk prefix over the W1 tiles (nw1 + 1), over the row tiles (n2 + 1),
+    // first chunk of every entry within its tile
+    DeviceBuffer<int> prefix;
+    DeviceBuffer<WideChunk> chunks;   // wide: the chunks of phase 1, then of phase 2
     int nw1 = 0;
     long long wc1 = 0, wc2 = 0;     // wide: chunks of phase 1 / phase 2
     // Host copies, and per split width GW the first item / (tile, entry) of
