@@ -31,6 +31,7 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
+constexpr int kCtasPerSm = 2;   // (launch bound of the blocks kernel)
 constexpr int kMaxRows = 512;   // rows (or input rows) of one warp unit
 constexpr int kMaxRank = 128;   // larger ranks use the general kernels
 constexpr int kWaitLimit = 1 << 24;
@@ -258,7 +259,7 @@ struct MvArgs {
     int nunits, nbig, nwarps;
 };
 
-__global__ void __launch_bounds__(kThreads, 2) mv_blocks_kernel(const MvArgs a) {
+__global__ void __launch_bounds__(kThreads, kCtasPerSm) mv_blocks_kernel(const MvArgs a) {
     __shared__ double ts[kWarps][kMaxRank];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double* t = ts[warp];
@@ -439,6 +440,24 @@ std::shared_ptr<MvPlan> build_plan(Context& ctx, const HMatrix& H, int root, boo
             }
         }
     }
+    // Dense leaves are cut where the matrix has too few blocks to occupy the
+    // warps twice: one warp takes a 170 x 170 leaf in 85 dependent steps of two
+    // columns, six warps with 32 rows each in 11 of sixteen.  A unit then holds
+    // at least its share of the data, so that matrices with many blocks (whose
+    // bound is HBM, which wants long contiguous runs) keep whole leaves.
+    // Slabs are multiples of 32 rows (of 16 columns for the transpose), which
+    // leaves every sum in its order.  58 x 47 grid, 3 levels (170-point
+    // leaves), rank 19: 68 -> 21 us,
+    // 170 x 150 grid, 6 levels: 69 us either way.
+    long long stored = 0;
+    for (int b : leaves) {
+        const Block& B = S.blocks[b];
+        stored += B.kind == KIND_DENSE ? (long long)B.m * B.n : (long long)(B.m + B.n) * H.rank[b];
+    }
+    const long long share = std::max(1LL, stored / (2LL * kCtasPerSm * kWarps * ctx.num_sms));
+    auto slab_of = [&](long long other, int grain) {
+        return (int)std::max<long long>(grain, share / std::max(1LL, other) / grain * grain);
+    };
     auto P = std::make_shared<MvPlan>();
     std::vector<MvUnit> first, rest;
     std::vector<MvBig> bigs;
@@ -470,9 +489,15 @@ std::shared_ptr<MvPlan> build_plan(Context& ctx, const HMatrix& H, int root, boo
                 u.r = nout;
             }
             u.in_off = in_off;
-            u.y_off = part;
             if (!cover(out0, out0 + nout)) return nullptr;
-            rest.push_back(u);
+            const int slab = slab_of(nin, trans ? 16 : 32);
+            for (int a0 = 0; a0 < nout; a0 += slab) {
+                MvUnit piece = u;
+                (trans ? piece.r : piece.rows_out) = std::min(slab, nout - a0);
+                piece.m1 += trans ? (long long)a0 * B.m : a0;
+                piece.y_off = part + a0;
+                rest.push_back(piece);
+            }
             part += nout;
             continue;
         }

@@ -71,3 +71,21 @@ def test_empty_and_errors(ctx):
     assert out.shape == (H.Height(), 0)
     with pytest.raises(D.HMError):
         H.Multiply(1.0, np.zeros(H.Width() + 1))
+
+
+@pytest.mark.parametrize("sizes,L,r", [((60, 60), 3, 5), ((32, 32), 3, 8), ((12, 12), 3, 2),
+                                       ((40, 40), 2, 3)])
+def test_one_vector_large_leaves(sizes, L, r):
+    """Few, large leaves (their rows are shared out among warps; grids that
+    halve evenly, as SetToRandom needs): remainders of
+    32 rows and of 16 columns, blocks below one slab, a tree of dense leaves only."""
+    from oracle import dmhm_oracle as O
+    c = D.Context(0)
+    coef = D.operators.uniform_coefficients(sizes, 6)
+    H = D.HMat2d(D.operators.stencil(sizes, coef, L), L, r, True, *sizes, ctx=c)
+    H.SetToRandom()
+    Ho = O.build_stencil_hmat(2, sizes, L, r, coef)
+    O.set_to_random(Ho, O.Rng())
+    x = np.random.default_rng(8).standard_normal(sizes[0] * sizes[1])
+    assert relerr(H.Multiply(1.0, x), O.multiply_dense(Ho, 1.0, x[:, None])[:, 0]) < 1e-13
+    assert relerr(H.TransposeMultiply(1.0, x), O.transpose_multiply_dense(Ho, 1.0, x[:, None])[:, 0]) < 1e-13
