@@ -30,8 +30,9 @@ void upload_gemm_tiles(Context& ctx, const std::vector<GemmOp>& ops, GemmTileLis
 void launch_gemm_tiles(Context& ctx, const GemmTileList& L, const RelocBases& bases,
                        const char* name);
 
-// One CTA per worker w running ops [begin[w], begin[w+1]) in order (ops of one
-// worker may update the same C); different workers write disjoint C.
+// One CTA per worker w and 64 x 64 tile of its C, running ops [begin[w],
+// begin[w+1]) in order (all ops of a worker update one C); different workers
+// write disjoint C, and no op reads another's C.
 void launch_gemm_workers(Context& ctx, const std::vector<GemmOp>& ops,
                          const std::vector<int>& begin, const char* name);
 // The same from a device-resident list whose pointers may be tagged offsets
@@ -39,7 +40,7 @@ void launch_gemm_workers(Context& ctx, const std::vector<GemmOp>& ops,
 struct GemmList {
     DeviceBuffer<GemmOp> ops;
     DeviceBuffer<int> begin;
-    int nw = 0;
+    int nw = 0, tiles = 1;   // 64 x 64 tiles of the largest C
 };
 void upload_gemm_list(Context& ctx, const std::vector<GemmOp>& ops, const std::vector<int>& begin,
                       GemmList& out);
