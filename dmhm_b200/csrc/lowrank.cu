@@ -96,8 +96,6 @@ __device__ __forceinline__ R warp_sum(R v) {
 namespace hmb {
 namespace {
 
-constexpr int kRegCols = 96;   // most columns of an op of the register form
-
 template <typename R>
 __device__ R block_sum(R v, R* red) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -802,25 +800,6 @@ void launch_round_typed(Context& ctx, const RoundList& L, const RelocBases& base
 
 namespace {
 
-int op_columns(const RoundOp& op) {
-    return op.kind == ROUND_DENSE ? op.n : op.r1 + (op.kind == ROUND_GENERAL ? op.r2 : 0);
-}
-
-// Warps the register form (round_reg.cuh) needs to hold an op: 4 or 8; 16 when
-// its stacks do not fit (the general kernel runs the worker then).  Small ops
-// would fit 1 or 2 warps, but every step waits for the same chain of
-// operations whatever its width, and one kernel for all ops of a list shares
-// the instruction cache (64 x 64 blocks of rank 16, whole product: 16.0 ms;
-// with 1 and 2 warps where they fit 18.8 ms, with 8 warps for all 24 ms).
-int reg_warps(const RoundOp& op, bool fp32) {
-    if (op.kind == ROUND_SET || op.kind == ROUND_CONCAT) return 4;
-    const int cols = std::max(op_columns(op), op.rout);
-    if (cols > kRegCols) return 16;
-    for (int nw = 4; nw <= 8; nw *= 2)
-        if (std::max(std::max(op.m, op.n), cols) <= reground::slab_rows(cols, nw, fp32)) return nw;
-    return 16;
-}
-
 // Relative time of an op, for the order in which workers start.
 double op_cost(const RoundOp& op) {
     if (op.kind == ROUND_SET || op.kind == ROUND_CONCAT) return 0.1 * op.rout;
@@ -874,7 +853,7 @@ void schedule(const std::vector<RoundOp>& ops, const std::vector<int>& begin,
         for (int i = G.first; i < G.first + G.count; ++i)
             for (int o = begin[index[base + i]]; o < begin[index[base + i] + 1]; ++o) {
                 if (ops[o].kind == ROUND_SET || ops[o].kind == ROUND_CONCAT) continue;
-                G.cols = std::max(G.cols, std::max(op_columns(ops[o]), ops[o].rout));
+                G.cols = std::max(G.cols, layout_columns(ops[o]));
                 G.rout = std::max(G.rout, ops[o].rout);
             }
     }

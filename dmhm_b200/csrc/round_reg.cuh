@@ -29,39 +29,12 @@
 // 924 -> 221 ms in 36; FP32, 72 x 68 grid, 765 -> 192 ms in 28.
 #pragma once
 
-#include "lowrank.h"
+#include "round_sizing.h"
 
 namespace hmb {
 namespace reground {
 
-constexpr int kSlabMax = 64;    // rows of a slab
-constexpr int kChunk = 4;       // inner products exchanged per barrier in step 6
 constexpr int kMaxSweeps = 40;
-
-// Shared memory of a CTA of NW warps whose ops have at most `cols` columns
-// (stacked rank or dense width) and `rout` output columns.  Passed by value and
-// addressed from the shared array in every function, so that the accesses stay
-// shared-memory ones and the offsets stay in registers.
-struct Layout {
-    int cp, rp, ld, rows;   // padded columns, output columns; matrix ld, rows
-    int part, rowt, chunk, tau, nrm, jex, order, mat, total;
-    __host__ __device__ Layout(int nw, int cols, int rout)
-        : cp((cols + 31) & ~31), rp((rout + 31) & ~31),
-          ld((cols > rp ? cols : rp) | 1), rows((cols + 1) & ~1) {
-        part = 2 * nw * kSlabMax;                 // us: 2 x nw x 64
-        rowt = part + 3 * nw * cp;                // part: 3 x nw x cp
-        tau = rowt + 2 * cp;                      // rowt: 2 x cp
-        // the exchange buffers of the sweeps (jex: 2 x nw x 32) and of step 6
-        // (chunk: 2 x nw x kChunk x rp) take the place of part and rowt
-        chunk = jex = part;
-        const int other = part + 2 * nw * (kChunk * rp > 32 ? kChunk * rp : 32);
-        if (other > tau) tau = other;
-        nrm = tau + cp;
-        order = nrm + cp + 2;                     // nrm: cp + 2
-        mat = (order + cp + 4 + 1) & ~1;          // order (ints) and one flag
-        total = mat + rows * ld + 2;
-    }
-};
 
 template <typename R>
 __device__ __forceinline__ R* shared_base() {
@@ -940,16 +913,6 @@ __device__ __noinline__ void phase_v(const Cta<R, NW> C, const Stack& V, int rou
             else { CALL(3, (wide_ ? 24 : 12)); }                              \
         }                                                                     \
     } while (0)
-
-// Rows that nw warps hold for `cols` columns (0: more columns than any slab).
-// A lane's share of a slab takes 64 registers at most, so that the broadcast
-// reads of a step stay in flight beside it and 16 warps share an SM: twice the
-// rows (half the warps) took 14 % longer on 64 x 64 blocks of rank 16 and
-// 40 % longer on 72-row complex ones.
-__host__ __device__ inline int slab_rows(int cols, int nw, bool fp32) {
-    const int rows = cols <= 32 ? 32 : cols <= 64 ? 16 : cols <= 96 ? 12 : 0;
-    return nw * (fp32 ? 2 * rows : rows);
-}
 
 // One GENERAL, DENSE or ORTHO rounding by the whole CTA.
 template <typename R, int NW>

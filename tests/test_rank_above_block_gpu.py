@@ -1,0 +1,85 @@
+"""Blocks whose stored rank exceeds their size (legal in an unpacked matrix:
+any rank >= 0) as the state that a dense x dense compression of an H*H product
+adds to, from ranks just above the block to past the register form's columns.
+The products are exact (ranks up to the block size are kept), so they agree
+with dense algebra to rounding."""
+import struct
+
+import numpy as np
+import pytest
+
+import dmhm_b200 as D
+from helpers import relerr
+
+pytestmark = pytest.mark.gpu
+SIDE, LEVELS = 16, 3          # 16 leaf boxes of 16 points
+
+
+def boxes(level):
+    """(coordinates, offset, points) of the boxes of a level, depth first."""
+    out = [((0, 0), 0, SIDE * SIDE)]
+    for _ in range(level):
+        out = [((2 * c[0] + (q & 1), 2 * c[1] + (q >> 1)), o + q * n // 4, n // 4)
+               for c, o, n in out for q in range(4)]
+    return out
+
+
+def pack(maxrank, dense, low):
+    """Wire format of a matrix with the given leaf blocks: dense[(t, s)] and
+    low[(t, s)] = (U, V) by leaf coordinates; absent dense blocks are zero,
+    absent low-rank blocks empty."""
+    out = [struct.pack("=iiii??", LEVELS, maxrank, 0, 0, False, True),
+           struct.pack("=iiii", SIDE, SIDE, SIDE, SIDE), struct.pack("=iiii", 0, 0, 0, 0)]
+
+    def walk(t, s, level):
+        if max(abs(a - b) for a, b in zip(t, s)) > 1:
+            U, V = low.get((t, s), (np.zeros((0, 0)), np.zeros((0, 0))))
+            out.append(struct.pack("=ii", 2, U.shape[1]) + U.T.tobytes() + V.T.tobytes())
+        elif level < LEVELS - 1:
+            out.append(struct.pack("=i", 0))
+            kids = [[(2 * b[0] + (q & 1), 2 * b[1] + (q >> 1)) for q in range(4)] for b in (t, s)]
+            for tc in kids[0]:
+                for sc in kids[1]:
+                    walk(tc, sc, level + 1)
+        else:
+            d = dense.get((t, s), np.zeros((16, 16)))
+            out.append(struct.pack("=ii", 3, 0) + np.ascontiguousarray(d.T).tobytes())
+
+    walk((0, 0), (0, 0), 0)
+    return b"".join(out) + b"\0" * 4
+
+
+def full(dense, low):
+    at = {c: o for c, o, _ in boxes(LEVELS - 1)}
+    M = np.zeros((SIDE * SIDE, SIDE * SIDE))
+    for (t, s), d in dense.items():
+        M[at[t]:at[t] + 16, at[s]:at[s] + 16] = d
+    for (t, s), (U, V) in low.items():
+        M[at[t]:at[t] + 16, at[s]:at[s] + 16] = U @ V.T
+    return M
+
+
+@pytest.mark.parametrize("rank", [17, 20, 33, 64, 96, 97, 130])
+@pytest.mark.parametrize("low_precision", [False, True])
+def test_dense_compression_onto_a_rank_above_the_block(rank, low_precision):
+    rng = np.random.default_rng(rank)
+    leaf = [c for c, _, _ in boxes(LEVELS - 1)]
+    near = [(t, s) for t in leaf for s in leaf if max(abs(a - b) for a, b in zip(t, s)) <= 1]
+    da = {ts: rng.standard_normal((16, 16)) for ts in near}
+    db = {ts: rng.standard_normal((16, 16)) for ts in near}
+    la = {((2, 0), (0, 0)): (rng.standard_normal((16, rank)), rng.standard_normal((16, rank)))}
+    c = D.Context(0)
+    c.set_low_precision(low_precision)
+    A = D.HMat2d.Unpack(pack(rank, da, la), ctx=c)
+    B = D.HMat2d.Unpack(pack(rank, db, {}), ctx=c)
+    a, b = full(da, la), full(db, {})
+    P = rng.standard_normal((SIDE * SIDE, 4))
+    assert relerr(A.Multiply(1.0, P), a @ P) < 1e-13
+    # FP64: a few roundings of 1e-15 each; FP32: its sweeps stop at couplings of 1e-6
+    tol = 1e-5 if low_precision else 1e-12
+    assert relerr(A.Multiply(1.0, B).Multiply(1.0, P), a @ (b @ P)) < tol
+    if rank > 64:       # (an update stacks 2 rank columns, 128 at most)
+        return
+    X = D.HMat2d(ctx=c).CopyFrom(A)
+    A.Multiply(0.5, B, -0.7, X)
+    assert relerr(X.Multiply(1.0, P), 0.5 * (a @ (b @ P)) - 0.7 * (a @ P)) < tol
