@@ -9,6 +9,8 @@
 
 #include <algorithm>
 
+#include "kernel_limits.h"
+
 namespace hmb {
 
 namespace {
@@ -286,11 +288,6 @@ gemm_worker_kernel(const GemmOp* __restrict__ ops, const int* __restrict__ begin
     if (tile < tm * tn) gemm_tile(ops, b0, b1, (tile % tm) * 64, (tile / tm) * 64, bases, gemm_smem);
 }
 
-template <typename K>
-void allow_smem(K kernel) {
-    HMB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
-}
-
 }  // namespace
 
 void upload_gemm_tiles(Context& ctx, const std::vector<GemmOp>& ops, GemmTileList& out) {
@@ -315,7 +312,7 @@ void upload_gemm_tiles(Context& ctx, const std::vector<GemmOp>& ops, GemmTileLis
 void launch_gemm_tiles(Context& ctx, const GemmTileList& L, const RelocBases& bases,
                        const char* name) {
     if (L.ntiles == 0) return;
-    allow_smem(gemm_ops_kernel);
+    allow_smem(gemm_ops_kernel, kSmem);
     LaunchScope ls(ctx, name);
     gemm_ops_kernel<<<(unsigned)L.ntiles, kT, kSmem, ctx.stream>>>(L.ops.get(), L.tile_op.get(),
                                                                L.tile_id.get(), bases);
@@ -341,7 +338,7 @@ void upload_gemm_list(Context& ctx, const std::vector<GemmOp>& ops, const std::v
 
 void launch_gemm_list(Context& ctx, const GemmList& L, const RelocBases& bases, const char* name) {
     if (L.nw == 0) return;
-    allow_smem(gemm_worker_kernel);
+    allow_smem(gemm_worker_kernel, kSmem);
     LaunchScope ls(ctx, name);
     gemm_worker_kernel<<<dim3((unsigned)L.nw, (unsigned)L.tiles), kT, kSmem, ctx.stream>>>(L.ops.get(), L.begin.get(), bases);
     HMB_CHECK_LAUNCH();

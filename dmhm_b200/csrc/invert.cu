@@ -20,10 +20,9 @@
 // compression the draws the reference's sequence of Multiply calls gives
 // it.  Factors that would alias the output are read from a copy.
 #include <algorithm>
-#include <mutex>
-#include <set>
 
 #include "hh.h"
+#include "kernel_limits.h"
 #include "schulz.h"
 
 namespace hmb {
@@ -99,18 +98,7 @@ void invert_dense_leaf(Context& ctx, HMatrix& X, int b) {
                 "DirectInvert handles dense leaves of at most 96 rows");
     if (B.m == 0) return;
     const size_t smem = (size_t)B.m * 2 * B.m * sizeof(double);
-    {
-        // once per device (contexts on several host threads may get here at once)
-        int dev = 0;
-        HMB_CUDA(cudaGetDevice(&dev));
-        static std::mutex mu;
-        static std::set<int> done;
-        std::lock_guard<std::mutex> lock(mu);
-        if (done.insert(dev).second)
-            HMB_CUDA(cudaFuncSetAttribute(
-                invert_leaf_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                (int)(kMaxLeafInvert * 2 * kMaxLeafInvert * sizeof(double))));
-    }
+    allow_smem(invert_leaf_kernel, kMaxLeafInvert * 2 * kMaxLeafInvert * sizeof(double));
     X.shadow_valid = false;
     LaunchScope ls(ctx, "invert_leaf");
     invert_leaf_kernel<<<1, kInvThreads, smem, ctx.stream>>>(X.D(b), B.m, ctx.numerical_word());

@@ -27,9 +27,8 @@
 #include "lowrank.h"
 
 #include <algorithm>
-#include <map>
-#include <mutex>
-#include <utility>
+
+#include "kernel_limits.h"
 
 namespace hmb {
 
@@ -738,20 +737,6 @@ void launch_round_ops(Context& ctx, std::vector<RoundOp>& ops, const char* name)
 
 
 namespace {
-
-// Once per device (contexts on several host threads may get here at once).
-template <typename K>
-void allow_smem(K kernel, size_t bytes) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    static std::mutex mu;
-    static std::map<std::pair<int, const void*>, size_t> done;
-    std::lock_guard<std::mutex> lock(mu);
-    size_t& have = done[{dev, reinterpret_cast<const void*>(kernel)}];
-    if (have >= bytes) return;
-    HMB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-    have = bytes;
-}
 
 template <typename R, int NW>
 void launch_round_reg(const RoundList& L, const int* workers, const RoundList::Group& g,

@@ -23,9 +23,9 @@
 #include <type_traits>
 #include <cstring>
 #include <map>
-#include <mutex>
 
 #include "engine.h"
+#include "kernel_limits.h"
 #include "templates.h"
 
 namespace hmb {
@@ -1380,30 +1380,8 @@ namespace {
 
 // Resident CTAs of a persistent kernel of `threads` threads a CTA.
 template <typename K>
-int persistent_grid_n(const Context& ctx, K kernel, int threads, size_t smem = 0) {
-    static std::mutex mu;
-    static std::map<const void*, int> per_sm;
-    std::lock_guard<std::mutex> lock(mu);
-    int& n = per_sm[(const void*)kernel];
-    if (n == 0) {
-        HMB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem));
-        n = std::max(1, n);
-    }
-    return n * ctx.num_sms;
-}
-
-// Resident CTAs of a persistent kernel (occupancy x SMs), cached per kernel.
-template <typename K>
-int persistent_grid(const Context& ctx, K kernel) {
-    static std::mutex mu;
-    static std::map<const void*, int> per_sm;
-    std::lock_guard<std::mutex> lock(mu);
-    int& n = per_sm[(const void*)kernel];
-    if (n == 0) {
-        HMB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kThreads, 0));
-        n = std::max(1, n);
-    }
-    return n * ctx.num_sms;
+int persistent_grid(const Context& ctx, K kernel, int threads, size_t smem = 0) {
+    return ctas_per_sm(kernel, threads, smem) * ctx.num_sms;
 }
 
 // First item of every warp of the narrow phase-1 kernel for split width GW.
@@ -1447,7 +1425,7 @@ void launch_narrow(Context& ctx, const JobExec* jobs_d, int nj, const JobExec& j
     cudaStream_t st = ctx.stream;
     if (c1 > 0) {
         const long long g = std::min<long long>(ceil_div(c1, kWarps),
-                                                persistent_grid(ctx, p1_stream_kernel<NC>));
+                                                persistent_grid(ctx, p1_stream_kernel<NC>, kThreads));
         const long long GW = std::min<long long>(g * kWarps, c1);
         const int* starts = single ? warp_starts1(ctx, *single, GW) : nullptr;
         DeviceBuffer<double> S;
@@ -1459,7 +1437,7 @@ void launch_narrow(Context& ctx, const JobExec* jobs_d, int nj, const JobExec& j
     }
     if (c2 > 0) {
         const long long g = std::min<long long>(ceil_div(c2, kWarps),
-                                                persistent_grid(ctx, p2_stream_kernel<NC>));
+                                                persistent_grid(ctx, p2_stream_kernel<NC>, kThreads));
         const long long GW = std::min<long long>(g * kWarps, c2);
         const int2* starts = single ? warp_starts2(ctx, *single, GW) : nullptr;
         DeviceBuffer<double> S;
@@ -1491,13 +1469,9 @@ __global__ void in_tf32_kernel(const InConv* __restrict__ cv) {
 // Grids and launches of the FP64 tiles (NT columns a tile).
 template <int PHASE, int NT, bool ONE>
 int wide64_grid(Context& ctx, long long chunks) {
-    static std::once_flag attr_once;
-    std::call_once(attr_once, [] {
-        cudaFuncSetAttribute(wide64_kernel<PHASE, NT, ONE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)Tile64<NT>::smem);
-    });
+    allow_smem(wide64_kernel<PHASE, NT, ONE>, Tile64<NT>::smem);
     return (int)std::min<long long>(
-        chunks, persistent_grid_n(ctx, wide64_kernel<PHASE, NT, ONE>, WTHREADS, Tile64<NT>::smem));
+        chunks, persistent_grid(ctx, wide64_kernel<PHASE, NT, ONE>, WTHREADS, Tile64<NT>::smem));
 }
 
 // f(integral_constant<NT>) for nt = 8, 16, 32 or 64.
@@ -1543,13 +1517,10 @@ void launch_wide64(Context& ctx, int nt, const JobExec* jobs_d, int nj, const Jo
 
 void wide_tf32_grids(Context& ctx, long long c1, long long c2, int& G1, int& G2) {
     constexpr size_t smem = sizeof(WideSmem32);
-    static std::once_flag attr_once;
-    std::call_once(attr_once, [] {
-        cudaFuncSetAttribute(wide_tf32_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        cudaFuncSetAttribute(wide_tf32_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    });
-    G1 = (int)std::min<long long>(c1, persistent_grid_n(ctx, wide_tf32_kernel<1>, WTHREADS, smem));
-    G2 = (int)std::min<long long>(c2, persistent_grid_n(ctx, wide_tf32_kernel<2>, WTHREADS, smem));
+    allow_smem(wide_tf32_kernel<1>, smem);
+    allow_smem(wide_tf32_kernel<2>, smem);
+    G1 = (int)std::min<long long>(c1, persistent_grid(ctx, wide_tf32_kernel<1>, WTHREADS, smem));
+    G2 = (int)std::min<long long>(c2, persistent_grid(ctx, wide_tf32_kernel<2>, WTHREADS, smem));
 }
 
 void launch_wide_tf32(Context& ctx, const JobExec* jobs_d, int nj, const JobExec& job0, long long n1,

@@ -20,9 +20,9 @@
 #include <algorithm>
 #include <map>
 #include <memory>
-#include <mutex>
 
 #include "engine.h"
+#include "kernel_limits.h"
 #include "templates.h"
 
 namespace hmb {
@@ -604,12 +604,7 @@ bool multiply_vector_streamed(Context& ctx, const MatJob& J) {
     if (P.nunits == 0) return false;
     cudaStream_t st = ctx.stream;
     int* cnt = ctx.zeroed_counters(2 + P.nbig);
-    static std::once_flag once;
-    static int per_sm = 0;
-    std::call_once(once, [] {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mv_blocks_kernel, kThreads, 0);
-        per_sm = std::max(1, per_sm);
-    });
+    const int per_sm = ctas_per_sm(mv_blocks_kernel, kThreads);
     const int g = std::max(1, std::min(per_sm * ctx.num_sms, (P.nunits + kWarps - 1) / kWarps));
     MvArgs a{};
     a.hb = J.H->data.get();
