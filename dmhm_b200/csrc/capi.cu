@@ -104,6 +104,15 @@ void Context::join(int n) {
     }
 }
 
+void Context::drain(int n) noexcept {
+    for (int i = 0; i < n; ++i)
+        if (cudaEventRecord(side_done[i], side[i]) != cudaSuccess ||
+            cudaStreamWaitEvent(stream, side_done[i], 0) != cudaSuccess) {
+            cudaGetLastError();   // (the error that ended the scope is reported)
+            cudaStreamSynchronize(side[i]);
+        }
+}
+
 void Context::release_side() {
     for (int i = 0; i < kSideStreams; ++i) {
         if (side[i]) cudaStreamDestroy(side[i]);

@@ -102,12 +102,15 @@ struct Context {
     // Side streams for launches that are independent of one another: fork()
     // makes `n` of them wait for the work queued on `stream` so far, join()
     // makes `stream` wait for theirs, so that everything queued on `stream`
-    // afterwards (frees included) follows it.  Made on first use.
+    // afterwards (frees included) follows it; drain() does that without
+    // throwing, waiting on the host where it must.  Used through ForkScope
+    // (fork_scope.h).  Made on first use.
     static constexpr int kSideStreams = 4;
     cudaStream_t side[kSideStreams] = {};
     cudaEvent_t side_fork = nullptr, side_done[kSideStreams] = {};
     void fork(int n);
     void join(int n);
+    void drain(int n) noexcept;
     void release_side();
     // Device word set by kernels whose bounded waits gave up (zero = fine);
     // read and cleared by check_numerical().

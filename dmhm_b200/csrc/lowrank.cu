@@ -28,6 +28,7 @@
 
 #include <algorithm>
 
+#include "fork_scope.h"
 #include "kernel_limits.h"
 
 namespace hmb {
@@ -739,11 +740,14 @@ void launch_round_ops(Context& ctx, std::vector<RoundOp>& ops, const char* name)
 namespace {
 
 template <typename R, int NW>
+size_t round_reg_smem(const RoundList::Group& g) {
+    return (size_t)reground::Layout(NW, g.cols, g.rout).total * sizeof(R);
+}
+
+template <typename R, int NW>
 void launch_round_reg(const RoundList& L, const int* workers, const RoundList::Group& g,
                       const RelocBases& bases, int* numflag, cudaStream_t st) {
-    const size_t bytes = (size_t)reground::Layout(NW, g.cols, g.rout).total * sizeof(R);
-    allow_smem(round_reg_kernel<R, NW>, bytes);
-    round_reg_kernel<R, NW><<<(unsigned)g.count, NW * 32, bytes, st>>>(
+    round_reg_kernel<R, NW><<<(unsigned)g.count, NW * 32, round_reg_smem<R, NW>(g), st>>>(
         L.ops.get(), L.index.get(), workers + g.first, g.cols, g.rout, bases, numflag);
     HMB_CHECK_LAUNCH();
 }
@@ -759,13 +763,19 @@ void launch_round_typed(Context& ctx, const RoundList& L, const RelocBases& base
     int parts = sch.nw_general > 0 ? 1 : 0;
     for (const RoundList::Group& g : sch.groups) parts += g.count > 0 ? 1 : 0;
     if (parts == 0) return;
+    if (sch.nw_general > 0)
+        allow_smem(round_worker_kernel<R>, (size_t)(sizeof(R) == 8 ? kSmemBytes : kSmemBytesF32));
+    for (const RoundList::Group& g : sch.groups) {
+        if (g.count == 0) continue;
+        if (g.warps == 4) allow_smem(round_reg_kernel<R, 4>, round_reg_smem<R, 4>(g));
+        else allow_smem(round_reg_kernel<R, 8>, round_reg_smem<R, 8>(g));
+    }
     LaunchScope ls(ctx, name);
     g_launches.fetch_add(parts - 1, std::memory_order_relaxed);
-    if (parts > 1) ctx.fork(parts - 1);
+    ForkScope<Context> fork(ctx, parts - 1);
     int next = 0;   // the first part stays on the context's stream
     auto stream = [&]() { return next++ == 0 ? ctx.stream : ctx.side[next - 2]; };
     if (sch.nw_general > 0) {
-        allow_smem(round_worker_kernel<R>, (size_t)(sizeof(R) == 8 ? kSmemBytes : kSmemBytesF32));
         round_worker_kernel<R><<<(unsigned)sch.nw_general, kT, sch.smem * sizeof(R), stream()>>>(
             L.ops.get(), L.index.get(), workers, sch.smem, bases, numflag);
         HMB_CHECK_LAUNCH();
@@ -773,12 +783,10 @@ void launch_round_typed(Context& ctx, const RoundList& L, const RelocBases& base
     for (const RoundList::Group& g : sch.groups) {
         if (g.count == 0) continue;
         const cudaStream_t st = stream();
-        switch (g.warps) {
-            case 4: launch_round_reg<R, 4>(L, workers, g, bases, numflag, st); break;
-            default: launch_round_reg<R, 8>(L, workers, g, bases, numflag, st); break;
-        }
+        if (g.warps == 4) launch_round_reg<R, 4>(L, workers, g, bases, numflag, st);
+        else launch_round_reg<R, 8>(L, workers, g, bases, numflag, st);
     }
-    if (parts > 1) ctx.join(parts - 1);
+    fork.join();
 }
 
 }  // namespace
