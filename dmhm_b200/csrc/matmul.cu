@@ -1031,36 +1031,50 @@ wide64_kernel(const JobExec* __restrict__ jobs, int njobs, const JobExec job0, l
         const W1Tile* wt = PHASE == 1 ? J.w1 + mt.y : nullptr;
         P2T it{};
         if (PHASE == 2) it = J.p2[mt.y];
+        // one row of the tile's blocks (m of this warp) to where it belongs
+        auto store_row = [&](int m, const double (&v)[NB][2]) {
+            const int i = 8 * (WM * m + wm) + g;
+            if (i >= trows) return;
+            long long rbase = 0, rstep = 0;
+            if (PHASE == 1) {
+                rbase = wt->trel[i] * J.k + wt->tj[i];
+                rstep = wt->tr[i];
+            }
+#pragma unroll
+            for (int c = 0; c < NB; ++c)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int col = 8 * (WN * c + wn) + 2 * t + h;
+                    if (col >= tcols) continue;
+                    if (PHASE == 1) J.T[rbase + (long long)(y * NT + col) * rstep] = v[c][h];
+                    else store_out(J, it, i, y * NT + col, v[c][h]);
+                }
+        };
         if (whole) {
 #pragma unroll
-            for (int m = 0; m < MB; ++m) {
-                const int i = 8 * (WM * m + wm) + g;
-                if (i >= trows) continue;
-                long long rbase = 0, rstep = 0;
-                if (PHASE == 1) {
-                    rbase = wt->trel[i] * J.k + wt->tj[i];
-                    rstep = wt->tr[i];
-                }
-#pragma unroll
-                for (int c = 0; c < NB; ++c)
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const int col = 8 * (WN * c + wn) + 2 * t + h;
-                        if (col >= tcols) continue;
-                        if (PHASE == 1) J.T[rbase + (long long)(y * NT + col) * rstep] = acc[m][c][h];
-                        else store_out(J, it, i, y * NT + col, acc[m][c][h]);
-                    }
-            }
+            for (int m = 0; m < MB; ++m) store_row(m, acc[m]);
         } else {
-            double* part = J.part + ((long long)y * 2 * G) * (WT * NT);
-            double* mine = part + (2LL * b + (first_piece ? 0 : 1)) * (WT * NT);
+            // Partials in the order of the accumulators, 16 bytes a thread; blocks
+            // beyond the tile are neither written nor read.  The last piece adds
+            // all of them in CTA order.  Bound by the latency of its loads, so
+            // several CTAs' partials are in flight for a block row, for the
+            // 8-column tiles for both block rows of a warp, within the registers
+            // of the main loop (whose spills cost more than this saves: all loads
+            // of four CTAs first, 8 columns of the 128 x 128 operator 114 us
+            // against 90).  One element after the other, 64 columns: 16 x 16
+            // points of rank 4 (16 pieces a tile) 141 -> 19 us, 128 x 128 points
+            // of rank 16 284 -> 227 us.
+            auto in_tile = [&](int m, int c) {
+                return 8 * (WM * m + wm) < trows && 8 * (WN * c + wn) < tcols;
+            };
+            double2* part = reinterpret_cast<double2*>(J.part) + ((long long)y * 2 * G) * (WT * NT / 2) + tid;
+            double2* mine = part + (2LL * b + (first_piece ? 0 : 1)) * (WT * NT / 2);
 #pragma unroll
             for (int m = 0; m < MB; ++m)
 #pragma unroll
                 for (int c = 0; c < NB; ++c)
-#pragma unroll
-                    for (int h = 0; h < 2; ++h)
-                        mine[8 * (WM * m + wm) + g + WT * (8 * (WN * c + wn) + 2 * t + h)] = acc[m][c][h];
+                    if (in_tile(m, c))
+                        mine[(m * NB + c) * WTHREADS] = make_double2(acc[m][c][0], acc[m][c][1]);
             __threadfence();
             __syncthreads();
             const long long wa = split_owner(T0, G, C), wb = split_owner(T1 - 1, G, C);
@@ -1070,15 +1084,30 @@ wide64_kernel(const JobExec* __restrict__ jobs, int njobs, const JobExec job0, l
             if (last_flag) {
                 __threadfence();
                 const bool wa_here = split_start(wa, G, C) == T0;
-                for (int o = tid; o < WT * tcols; o += WTHREADS) {
-                    const int i = o % WT, col = o / WT;
-                    if (i >= trows) continue;
-                    double v = 0.0;
-                    for (long long w = wa; w <= wb; ++w)
-                        v += __ldcg(part + piece_slot(w, wa, wa_here) * (WT * NT) + i + WT * col);
-                    if (PHASE == 1)
-                        J.T[wt->trel[i] * J.k + wt->tj[i] + (long long)(y * NT + col) * wt->tr[i]] = v;
-                    else store_out(J, it, i, y * NT + col, v);
+                constexpr int MG = NT == 8 ? MB : 1;   // block rows at a time
+#pragma unroll 1
+                for (int m0 = 0; m0 < MB && 8 * (WM * m0 + wm) < trows; m0 += MG) {
+                    double v[MG][NB][2];
+#pragma unroll
+                    for (int m = 0; m < MG; ++m)
+#pragma unroll
+                        for (int c = 0; c < NB; ++c) v[m][c][0] = v[m][c][1] = 0.0;
+#pragma unroll(NT == 16 ? 2 : 4)
+                    for (long long w = wa; w <= wb; ++w) {
+                        const double2* p =
+                            part + piece_slot(w, wa, wa_here) * (WT * NT / 2) + m0 * NB * WTHREADS;
+#pragma unroll
+                        for (int m = 0; m < MG; ++m)
+#pragma unroll
+                            for (int c = 0; c < NB; ++c)
+                                if (in_tile(m0 + m, c)) {
+                                    const double2 x = __ldcg(p + (m * NB + c) * WTHREADS);
+                                    v[m][c][0] += x.x;
+                                    v[m][c][1] += x.y;
+                                }
+                    }
+#pragma unroll
+                    for (int m = 0; m < MG; ++m) store_row(m0 + m, v[m]);
                 }
                 if (tid == 0) *cnt = 0;
             }
@@ -1798,7 +1827,8 @@ void run_jobs_direct(Context& ctx, const std::vector<MatJob>& jobs, bool tf32) {
             HMB_CHECK_LAUNCH();
         }
     }
-    tbuf.allocate((size_t)std::max<long long>((tf32 ? 0 : t_total) + p_total, 1), st);
+    const long long p_off = tf32 ? 0 : t_total + (t_total & 1);   // the partials on 16 bytes
+    tbuf.allocate((size_t)std::max<long long>(p_off + p_total, 1), st);
     int* cnt = ctx.zeroed_counters(std::max<long long>(c_total, 1));
     std::vector<JobExec> ex;
     ex.reserve(jobs.size());
@@ -1826,7 +1856,7 @@ void run_jobs_direct(Context& ctx, const std::vector<MatJob>& jobs, bool tf32) {
             e.part = tbuf.get();
         } else {
             e.T = tbuf.get() + t_off[j];
-            e.part = tbuf.get() + t_total;
+            e.part = tbuf.get() + p_off;
         }
         if (wide) {
             e.w1cp = T.prefix.get();
