@@ -91,7 +91,13 @@ void Context::fork(int n) {
     if (!side_fork) HMB_CUDA(cudaEventCreateWithFlags(&side_fork, cudaEventDisableTiming));
     HMB_CUDA(cudaEventRecord(side_fork, stream));
     for (int i = 0; i < n; ++i) {
-        if (!side[i]) HMB_CUDA(cudaStreamCreateWithFlags(&side[i], cudaStreamNonBlocking));
+        if (!side[i]) {
+            int least = 0, greatest = 0, base = 0;
+            HMB_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+            HMB_CUDA(cudaStreamGetPriority(stream, &base));
+            HMB_CUDA(cudaStreamCreateWithPriority(&side[i], cudaStreamNonBlocking,
+                                                  std::max(greatest, base - kSideStreams + i)));
+        }
         if (!side_done[i]) HMB_CUDA(cudaEventCreateWithFlags(&side_done[i], cudaEventDisableTiming));
         HMB_CUDA(cudaStreamWaitEvent(side[i], side_fork, 0));
     }

@@ -104,8 +104,10 @@ struct Context {
     // makes `stream` wait for theirs, so that everything queued on `stream`
     // afterwards (frees included) follows it; drain() does that without
     // throwing, waiting on the host where it must.  Used through ForkScope
-    // (fork_scope.h).  Made on first use.
-    static constexpr int kSideStreams = 4;
+    // (fork_scope.h).  Made on first use, each of a higher priority than the
+    // next and all of a higher one than `stream`, so that the CTAs of launches
+    // that become ready together start in the order side[0], side[1], `stream`.
+    static constexpr int kSideStreams = 2;
     cudaStream_t side[kSideStreams] = {};
     cudaEvent_t side_fork = nullptr, side_done[kSideStreams] = {};
     void fork(int n);

@@ -753,7 +753,11 @@ void launch_round_reg(const RoundList& L, const int* workers, const RoundList::G
 }
 
 // The groups of a list are independent (each worker writes its own block)
-// and each leaves SMs idle at its end, so they run at the same time.
+// and each leaves SMs idle at its end, so they run at the same time: those
+// with the longest CTAs first (the general kernel, then 8 warps), by the
+// priorities of the side streams.  Streams of one priority start in an order
+// that changes with the build: SchulzInvert mixed 72 x 68 took 330 ms or,
+// when the general kernel came last and ran on nearly alone, 378.
 template <typename R>
 void launch_round_typed(Context& ctx, const RoundList& L, const RelocBases& bases,
                         const char* name) {
@@ -773,8 +777,11 @@ void launch_round_typed(Context& ctx, const RoundList& L, const RelocBases& base
     LaunchScope ls(ctx, name);
     g_launches.fetch_add(parts - 1, std::memory_order_relaxed);
     ForkScope<Context> fork(ctx, parts - 1);
-    int next = 0;   // the first part stays on the context's stream
-    auto stream = [&]() { return next++ == 0 ? ctx.stream : ctx.side[next - 2]; };
+    int next = 0;   // the last part stays on the context's stream
+    auto stream = [&]() {
+        const int i = next++;
+        return i < parts - 1 ? ctx.side[i] : ctx.stream;
+    };
     if (sch.nw_general > 0) {
         round_worker_kernel<R><<<(unsigned)sch.nw_general, kT, sch.smem * sizeof(R), stream()>>>(
             L.ops.get(), L.index.get(), workers, sch.smem, bases, numflag);
