@@ -675,34 +675,54 @@ __device__ __noinline__ void jacobi_sweep(const Cta<R, NW> C, int n, int len, R 
         }
 }
 
-// The same sweep from shared memory for more than 64 columns: one warp a pair.
+// The same sweep from shared memory for 65 to 96 columns: eight lanes a pair,
+// twelve rows a lane, read once and rotated in registers.  A warp's four pairs
+// are NW apart, which with an odd ld puts their columns on the same banks
+// (FP64) or on different ones (FP32); rows are taken in an order that spreads
+// the former.
 template <typename R, int NW>
 __device__ __noinline__ void jacobi_sweep_wide(const Cta<R, NW> C, int n, int len, R tiny, R jt2) {
+    constexpr int RL = 12;   // rows of a lane: up to 96 rows
     R* mat = C.mat();
     R* nrm = C.nrm();
-    const int ld = C.L.ld;
+    const int ld = C.L.ld, grp = C.lane >> 3, hl = C.lane & 7;
+    const int turn = sizeof(R) == 8 ? grp & 1 : NW == 8 ? grp >> 1 : 0;
     for (int st = 0; st < n; ++st) {
-        for (int k = C.warp; 2 * k + 1 + (st & 1) < n; k += NW) {
-            const int p = 2 * k + (st & 1), q = p + 1;
+        const int np = (n - (st & 1)) >> 1;   // pairs of this step
+        for (int kb = 0; kb < np; kb += 4 * NW) {
+            const int k = kb + grp * NW + C.warp;
+            const bool live = k < np;
+            const int p = live ? 2 * k + (st & 1) : 0;
             R* gp = mat + p * ld;
-            R* gq = mat + q * ld;
-            R c = R(0);
-            for (int i = C.lane; i < len; i += 32) c = r_fma(gp[i], gq[i], c);
-            c = warp_sum(c);
-            const R nx = nrm[p], ny = nrm[q];
+            R* gq = gp + ld;
+            R x[RL], y[RL], cp[4] = {R(0), R(0), R(0), R(0)};
+#pragma unroll
+            for (int i = 0; i < RL; ++i) {
+                const int r = hl + 8 * (i ^ turn);
+                const bool v = live && r < len;
+                x[i] = v ? gp[r] : R(0);
+                y[i] = v ? gq[r] : R(0);
+                cp[i & 3] = r_fma(x[i], y[i], cp[i & 3]);
+            }
+            R c = (cp[0] + cp[1]) + (cp[2] + cp[3]);
+            const R nx = nrm[p], ny = nrm[p + 1];
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
             R cs = R(1), sn = R(0), tc = R(0);
             if (c != R(0) && nx > tiny && ny > tiny && c * c > jt2 * (nx * ny)) {
                 rotation(nx, ny, c, cs, sn, tc);
             }
-            for (int i = C.lane; i < len; i += 32) {
-                const R xi = gp[i], yi = gq[i];
-                gp[i] = r_fma(sn, xi, cs * yi);
-                gq[i] = r_fma(cs, xi, -(sn * yi));
+#pragma unroll
+            for (int i = 0; i < RL; ++i) {
+                const int r = hl + 8 * (i ^ turn);
+                if (live && r < len) {
+                    gp[r] = r_fma(sn, x[i], cs * y[i]);
+                    gq[r] = r_fma(cs, x[i], -(sn * y[i]));
+                }
             }
-            __syncwarp();
-            if (C.lane == 0) {
+            if (live && hl == 0) {   // (every lane has read the norms: the sum above)
                 nrm[p] = ny + tc;
-                nrm[q] = nx - tc;
+                nrm[p + 1] = nx - tc;
             }
         }
         __syncthreads();
