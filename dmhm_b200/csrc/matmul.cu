@@ -1120,6 +1120,63 @@ wide64_kernel(const JobExec* __restrict__ jobs, int njobs, const JobExec job0, l
     }
 }
 
+// The W1 tiles (CTAs 0 .. nw1 - 1) with their chunks, and the chunks of the row
+// tiles (the CTAs after them).
+__global__ void expand_template_kernel(const W1Source* __restrict__ src, int nw1, const P1T* __restrict__ p1,
+                                       const P2T* __restrict__ p2, int n2, const P2Entry* __restrict__ ent,
+                                       const int* __restrict__ prefix, W1Tile* __restrict__ w1,
+                                       WideChunk* __restrict__ chunks) {
+    const int* w1cp = prefix;
+    const int* tcp = prefix + nw1 + 1;
+    const int* ekc = tcp + n2 + 1;
+    const int tid = threadIdx.x, t = blockIdx.x;
+    if (t < nw1) {
+        const W1Source s = src[t];
+        W1Tile& w = w1[t];
+        if (tid == 0) {
+            w.in_off = s.in_off;
+            w.nin = s.nin;
+            w.rows = s.rows;
+        }
+        for (int i = tid; i < kWideTile; i += blockDim.x) {
+            long long wcol = 0, trel = 0;
+            int tj = 0, tr = 0;
+            if (i < s.rows) {
+                int it = s.item;
+                tj = s.col + i;
+                while (tj >= (tr = p1[it].r)) {
+                    tj -= tr;
+                    ++it;
+                }
+                wcol = p1[it].w + (long long)tj * p1[it].ldw;
+                trel = p1[it].t_rel;
+            }
+            w.wcol[i] = wcol;
+            w.trel[i] = trel;
+            w.tj[i] = tj;
+            w.tr[i] = tr;
+        }
+        WideChunk* c = chunks + w1cp[t];
+        for (int pos = tid * KC; pos < s.nin; pos += (int)blockDim.x * KC)
+            c[pos / KC] = {0, 0, (int)s.in_off, pos, 0, t,
+                           min(KC, s.nin - pos) | 256 | (pos + KC >= s.nin ? 512 : 0) | s.rows << 16};
+        return;
+    }
+    const int u = t - nw1;
+    const P2T it = p2[u];
+    for (int e = it.e0 + tid; e < it.e1; e += blockDim.x) {
+        const P2Entry E = ent[e];
+        WideChunk* c = chunks + w1cp[nw1] + tcp[u] + ekc[e];
+        for (int pos = 0; pos < E.inner; pos += KC) {
+            const long long a = E.a + (E.transA ? pos + (long long)it.r0 * E.lda
+                                                : it.r0 + (long long)pos * E.lda);
+            c[pos / KC] = {a, E.lda, (int)E.b_off, pos, E.b_from_t ? E.ldt : 0, u,
+                           min(KC, E.inner - pos) | (E.transA ? 256 : 0) |
+                               (e + 1 == it.e1 && pos + KC >= E.inner ? 512 : 0) | it.rows << 16};
+        }
+    }
+}
+
 // Work lists of one subtree of one H-matrix.
 std::shared_ptr<JobTemplate> build_template(Context& ctx, const HMatrix& H, int root,
                                             bool trans, int row_tile) {
@@ -1144,6 +1201,7 @@ std::shared_ptr<JobTemplate> build_template(Context& ctx, const HMatrix& H, int 
     }
     // phase 1 items
     std::vector<P1T> p1;
+    std::vector<int> p1_box;   // wide: source box of every item
     std::vector<long long> t_rel(leaves.size(), -1);
     long long t_rows = 0;
     for (size_t li = 0; li < leaves.size(); ++li) {
@@ -1167,6 +1225,7 @@ std::shared_ptr<JobTemplate> build_template(Context& ctx, const HMatrix& H, int 
         t_rel[li] = t_rows;
         t_rows += it.r;
         p1.push_back(it);
+        if (row_tile > 32) p1_box.push_back(trans ? B.tgt_box : B.src_box);
     }
     long long c1 = 0;
     int rmax = 0;
@@ -1177,32 +1236,40 @@ std::shared_ptr<JobTemplate> build_template(Context& ctx, const HMatrix& H, int 
     }
     // wide phase-1 tiles: the columns of the W's that share a source box
     // (one input slice), 64 to a tile
-    std::vector<W1Tile> w1;
+    std::vector<W1Source> w1;
     if (row_tile > 32) {
-        std::map<std::pair<long long, int>, std::vector<int>> groups;
-        for (int i = 0; i < (int)p1.size(); ++i) groups[{p1[i].in_off, p1[i].nin}].push_back(i);
-        for (auto& g : groups) {
-            W1Tile cur{};
-            cur.in_off = g.first.first;
-            cur.nin = g.first.second;
-            for (int i : g.second) {
-                for (int j = 0; j < p1[i].r; ++j) {
-                    if (cur.rows == kWideTile) {
-                        w1.push_back(cur);
-                        const long long io = cur.in_off;
-                        const int ni = cur.nin;
-                        cur = W1Tile{};
-                        cur.in_off = io;
-                        cur.nin = ni;
+        // by the source box's (offset, size): the few boxes sorted, the items counted in
+        std::vector<int> count(S.boxes.size() + 1, 0), boxes;
+        for (int b : p1_box)
+            if (count[b]++ == 0) boxes.push_back(b);
+        std::sort(boxes.begin(), boxes.end(), [&](int a, int b) {
+            return std::tie(S.boxes[a].offset, S.boxes[a].count, a) <
+                   std::tie(S.boxes[b].offset, S.boxes[b].count, b);
+        });
+        int at = 0;
+        for (int b : boxes) {
+            const int n = count[b];
+            count[b] = at;
+            at += n;
+        }
+        std::vector<P1T> sorted(p1.size());
+        for (size_t i = 0; i < p1.size(); ++i) sorted[count[p1_box[i]]++] = p1[i];
+        p1.swap(sorted);
+        for (size_t i = 0; i < p1.size();) {
+            const long long in_off = p1[i].in_off;
+            const int nin = p1[i].nin;
+            int rows = 0;   // of the group's last tile
+            for (; i < p1.size() && p1[i].in_off == in_off && p1[i].nin == nin; ++i)
+                for (int j = 0; j < p1[i].r;) {
+                    if (rows % kWideTile == 0) {
+                        w1.push_back({in_off, (int)i, j, 0, nin});
+                        rows = 0;
                     }
-                    cur.wcol[cur.rows] = p1[i].w + (long long)j * p1[i].ldw;
-                    cur.trel[cur.rows] = p1[i].t_rel;
-                    cur.tj[cur.rows] = j;
-                    cur.tr[cur.rows] = p1[i].r;
-                    ++cur.rows;
+                    const int take = std::min(kWideTile - rows, p1[i].r - j);
+                    rows += take;
+                    w1.back().rows = rows;
+                    j += take;
                 }
-            }
-            if (cur.rows > 0) w1.push_back(cur);
         }
     }
     // phase 2: bucket the leaves by the output clusters they cover
@@ -1293,22 +1360,22 @@ std::shared_ptr<JobTemplate> build_template(Context& ctx, const HMatrix& H, int 
     T->n1 = (int)p1.size();
     T->n2 = (int)p2.size();
     T->t_rows = t_rows;
-    T->nz = (int)zero.size();
     T->c1 = c1;
     T->c2 = c2;
     T->rmax = rmax;
-    // (the wide kernels take the W1 tiles; tc_matmul.cu the items of the whole
-    // matrix)
-    if (row_tile <= 32 || (root == 0 && !trans)) T->p1.upload(p1, ctx.stream);
+    T->p1.upload(p1, ctx.stream);
     T->p2.upload(p2, ctx.stream);
     T->ent.upload(ent, ctx.stream);
     T->hzero = zero;
     T->nw1 = (int)w1.size();
-    T->w1.upload(w1, ctx.stream);
     if (row_tile > 32) {
         // chunk prefixes of the wide kernels (chunks of KC inner indices,
-        // none spanning two entries)
-        std::vector<int> w1cp(w1.size() + 1, 0), tcp(p2.size() + 1, 0), ekc(ent.size(), 0);
+        // none spanning two entries): over the W1 tiles, over the row tiles,
+        // then every entry's first chunk within its tile
+        std::vector<int> prefix(w1.size() + 1 + p2.size() + 1 + ent.size(), 0);
+        int* w1cp = prefix.data();
+        int* tcp = w1cp + w1.size() + 1;
+        int* ekc = tcp + p2.size() + 1;
         for (size_t i = 0; i < w1.size(); ++i) w1cp[i + 1] = w1cp[i] + ceil_div(w1[i].nin, KC);
         for (size_t t = 0; t < p2.size(); ++t) {
             int k = 0;
@@ -1318,33 +1385,25 @@ std::shared_ptr<JobTemplate> build_template(Context& ctx, const HMatrix& H, int 
             }
             tcp[t + 1] = tcp[t] + k;
         }
-        T->wc1 = w1cp.back();
-        T->wc2 = tcp.back();
-        w1cp.insert(w1cp.end(), tcp.begin(), tcp.end());
-        w1cp.insert(w1cp.end(), ekc.begin(), ekc.end());
-        T->prefix.upload(w1cp, ctx.stream);
-        std::vector<WideChunk> ch;
-        ch.reserve((size_t)(T->wc1 + T->wc2));
-        for (size_t i = 0; i < w1.size(); ++i)
-            for (int pos = 0; pos < w1[i].nin; pos += KC) {
-                const int len = std::min(KC, w1[i].nin - pos);
-                ch.push_back({0, 0, (int)w1[i].in_off, pos, 0, (int)i,
-                              len | 256 | (pos + KC >= w1[i].nin ? 512 : 0) | w1[i].rows << 16});
-            }
-        for (size_t t = 0; t < p2.size(); ++t)
-            for (int e = p2[t].e0; e < p2[t].e1; ++e) {
-                const P2Entry& E = ent[e];
-                for (int pos = 0; pos < E.inner; pos += KC) {
-                    const int len = std::min(KC, E.inner - pos);
-                    const long long a = E.a + (E.transA ? pos + (long long)p2[t].r0 * E.lda
-                                                        : p2[t].r0 + (long long)pos * E.lda);
-                    ch.push_back({a, E.lda, (int)E.b_off, pos, E.b_from_t ? E.ldt : 0, (int)t,
-                                  len | (E.transA ? 256 : 0) |
-                                      (e + 1 == p2[t].e1 && pos + KC >= E.inner ? 512 : 0) |
-                                      p2[t].rows << 16});
-                }
-            }
-        T->chunks.upload(ch, ctx.stream);
+        T->wc1 = w1cp[w1.size()];
+        T->wc2 = tcp[p2.size()];
+        T->prefix.upload(prefix, ctx.stream);
+        // the tiles' columns and the chunks, made on the device: several times
+        // the bytes of the lists they come from (first product of 4 columns with
+        // a 128 x 128 operator of rank 4 to 13: 1950 us with lists from the host,
+        // 720 us)
+        T->w1.allocate(w1.size(), ctx.stream);
+        T->chunks.allocate((size_t)(T->wc1 + T->wc2), ctx.stream);
+        const size_t tiles = w1.size() + p2.size();
+        if (tiles > 0) {
+            DeviceBuffer<W1Source> src;
+            src.upload(w1, ctx.stream);
+            LaunchScope ls(ctx, "hmm_template_expand");
+            expand_template_kernel<<<(unsigned)tiles, 64, 0, ctx.stream>>>(
+                src.get(), (int)w1.size(), T->p1.get(), T->p2.get(), (int)p2.size(), T->ent.get(),
+                T->prefix.get(), T->w1.get(), T->chunks.get());
+            HMB_CHECK_LAUNCH();
+        }
     }
     T->hp1 = std::move(p1);
     T->hp2 = std::move(p2);

@@ -63,8 +63,15 @@ struct WideChunk {
     int bits;      // inner indices | inner-contiguous A << 8 | last of its tile << 9 | rows << 16
 };
 
+// What a W1Tile is made of: `rows` columns from column `col` of item `item` on,
+// through the items that follow (of one source box).
+struct W1Source {
+    long long in_off;
+    int item, col, rows, nin;
+};
+
 struct JobTemplate {
-    DeviceBuffer<P1T> p1;
+    DeviceBuffer<P1T> p1;           // (wide: grouped by source box)
     DeviceBuffer<P2T> p2;
     DeviceBuffer<P2Entry> ent;
     DeviceBuffer<W1Tile> w1;        // wide phase-1 tiles
@@ -87,7 +94,7 @@ struct JobTemplate {
     bool mv_tried = false;
     std::map<long long, DeviceBuffer<int>> start1;
     std::map<long long, DeviceBuffer<int2>> start2;
-    int n1 = 0, n2 = 0, nz = 0;
+    int n1 = 0, n2 = 0;
     long long c1 = 0, c2 = 0;       // rows of all items, columns of all tiles
     int rmax = 0;                   // largest rank among the items
     long long t_rows = 0;   // sum of the ranks: T holds t_rows * k entries
