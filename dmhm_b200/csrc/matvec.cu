@@ -18,7 +18,6 @@
 //     partial rows, in a fixed order) + beta * y_tile.
 // Deterministic: each partial is formed by exactly one warp in a fixed order.
 #include <algorithm>
-#include <map>
 #include <memory>
 
 #include "engine.h"
@@ -461,7 +460,7 @@ std::shared_ptr<MvPlan> build_plan(Context& ctx, const HMatrix& H, int root, boo
     auto P = std::make_shared<MvPlan>();
     std::vector<MvUnit> first, rest;
     std::vector<MvBig> bigs;
-    std::map<int, long long> yoff;   // block -> partial offset of its first output row
+    std::vector<long long> yoff(S.blocks.size(), -1);   // partial offset of a block's first output row
     std::vector<std::pair<int, int>> pcs;
     long long part = 0, tpart = 0;
     auto cover = [&](long long o0, long long o1) {
@@ -576,7 +575,7 @@ std::shared_ptr<MvPlan> build_plan(Context& ctx, const HMatrix& H, int root, boo
             const int b = T.hent_block[e];
             const Block& B = S.blocks[b];
             const long long out_row0 = trans ? B.col_off - R.col_off : B.row_off - R.row_off;
-            eo[e] = yoff.at(b) + (it.out_off - out_row0);
+            eo[e] = yoff[b] + (it.out_off - out_row0);
         }
     }
     P->units.upload(units, ctx.stream);
