@@ -188,19 +188,28 @@ __device__ void gemm_tile(const GemmOp* ops, int b0, int b1, int i0, int j0, con
         keep = 1.0;
     };
     bool pending = false;   // acc or keep hold something C does not
+    const int shift = m <= 8 ? 3 : m <= 16 ? 4 : m <= 32 ? 5 : 6;   // rows, as a power of two
     // an op without inner indices, in its turn
     auto plain = [&](int o) {
         const GemmOp op = resolve(ops[o], bases);
         if (pending) flush();
         pending = false;
         __syncthreads();   // C may be read by other threads than wrote it
-        for (int e = tid; e < 64 * 64; e += kT) {
-            const int i = e & 63, j = e >> 6;
-            if (i >= m || j >= n) continue;
-            const double a = op.k == 0 || op.alpha == 0.0
-                                 ? 0.0 : op.alpha * ld_op(op.A, op.lda, op.transA, i0 + i, j0 + j);
-            double* c = Cb + i + (long long)j * ldc;
-            *c = op.beta == 0.0 ? a : a + op.beta * *c;
+        const bool read = op.k != 0 && op.alpha != 0.0;
+        for (int e0 = tid; e0 < n << shift; e0 += 4 * kT) {
+            double a[4], v[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {   // all reads first: C may be A
+                const int e = e0 + q * kT, i = e & ((1 << shift) - 1), j = e >> shift;
+                const bool ok = i < m && j < n;
+                a[q] = ok && read ? op.alpha * ld_op(op.A, op.lda, op.transA, i0 + i, j0 + j) : 0.0;
+                v[q] = ok && op.beta != 0.0 ? Cb[i + (long long)j * ldc] : 0.0;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int e = e0 + q * kT, i = e & ((1 << shift) - 1), j = e >> shift;
+                if (i < m && j < n) Cb[i + (long long)j * ldc] = op.beta == 0.0 ? a[q] : a[q] + op.beta * v[q];
+            }
         }
         __syncthreads();
     };
