@@ -807,79 +807,133 @@ double op_cost(const RoundOp& op) {
     return k * (double)(op.m + op.n + 64);
 }
 
-// Appends one precision's worker list to `index`: by the kernel that runs
-// them, in the given order.
-void schedule(const std::vector<RoundOp>& ops, const std::vector<int>& begin,
-              const std::vector<int>& order, bool fp32, std::vector<int>& index,
-              RoundList::Schedule& out) {
-    const int nw = (int)begin.size() - 1;
-    std::vector<int> group(nw, 4);
-    for (int w = 0; w < nw; ++w)
-        for (int i = begin[w]; i < begin[w + 1]; ++i)
-            group[w] = std::max(group[w], reg_warps(ops[i], fp32));
-    out.workers = (int)index.size();
-    const int base = out.workers;
-    auto take = [&](auto pick) {
-        for (int w : order)
-            if (pick(group[w])) index.push_back(w);
-    };
-    take([](int need) { return need > 8; });
-    out.nw_general = (int)index.size() - base;
-    // General kernel: the core and the rotations of an op live in shared
-    // memory when they fit the launch's size, otherwise in the (L1-cached)
-    // global work area; the size is the largest need of its non-dense ops
-    // (dense compressions with larger cores take the global path), so that
-    // more CTAs share an SM.
+// The workers by falling cost, then by number: the longest operation lists
+// first, so that the last CTAs to start are short ones.
+std::vector<int> longest_first(const std::vector<double>& cost) {
+    const int nw = (int)cost.size();
+    std::vector<int> order(nw);
+    // blocks come in few sizes: counted by distinct cost (with this and one
+    // pass over the ops an update of 64 x 64 points, 5 levels, rank 2 takes 890
+    // us, with the workers sorted 1000)
+    constexpr int kDistinct = 32;
+    double value[kDistinct];
+    int count[kDistinct], rank[kDistinct], nd = 0;
+    std::vector<unsigned char> which(nw);
+    bool few = true;
+    for (int w = 0; w < nw && few; ++w) {
+        int d = w > 0 ? which[w - 1] : 0;   // (neighbours are often alike)
+        if (nd == 0 || value[d] != cost[w])
+            for (d = 0; d < nd && value[d] != cost[w]; ++d) {}
+        if (d == nd) {
+            few = nd < kDistinct;
+            if (!few) break;
+            value[nd] = cost[w];
+            count[nd++] = 0;
+        }
+        which[w] = (unsigned char)d;
+        ++count[d];
+    }
+    if (few) {
+        int at[kDistinct], next = 0;
+        for (int d = 0; d < nd; ++d) rank[d] = d;
+        std::sort(rank, rank + nd, [&](int a, int b) { return value[a] > value[b]; });
+        for (int i = 0; i < nd; ++i) {
+            at[rank[i]] = next;
+            next += count[rank[i]];
+        }
+        for (int w = 0; w < nw; ++w) order[at[which[w]]++] = w;
+        return order;
+    }
+    for (int w = 0; w < nw; ++w) order[w] = w;
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cost[a] > cost[b]; });
+    return order;
+}
+
+// One precision's part of a list: which kernel runs which worker, and the
+// shared memory of its launches.
+struct Scheduler {
+    bool fp32;
+    RoundList::Schedule& out;
+    std::vector<unsigned char> kernel;   // 0: general; 1, 2: register form, 8 and 4 warps
+    int count[3] = {0, 0, 0};
     long long need_max = 0;
-    for (int i = 0; i < out.nw_general; ++i)
-        for (int o = begin[index[base + i]]; o < begin[index[base + i] + 1]; ++o) {
-            const RoundOp& op = ops[o];
-            if (op.kind == ROUND_SET || op.kind == ROUND_CONCAT) continue;
-            const bool dense = op.kind == ROUND_DENSE;
-            const long long k = op_columns(op);
-            const long long ku = op.kind == ROUND_ORTHO ? op.r1 : std::min<long long>(op.m, k);
-            const long long kv = dense ? op.n : std::min<long long>(op.n, k);
+
+    Scheduler(bool fp32, RoundList::Schedule& out, size_t nw) : fp32(fp32), out(out) {
+        kernel.reserve(nw);
+        for (int g = 0; g < 2; ++g) out.groups[g] = RoundList::Group{8 >> g, 0, 0, 1, 1};
+    }
+    void add(const RoundOp* b, const RoundOp* e) {
+        int warps = 4;
+        for (const RoundOp* op = b; op < e; ++op) warps = std::max(warps, reg_warps(*op, fp32));
+        const int c = warps > 8 ? 0 : warps == 8 ? 1 : 2;
+        kernel.push_back((unsigned char)c);
+        ++count[c];
+        for (const RoundOp* op = b; op < e; ++op) {
+            if (op->kind == ROUND_SET || op->kind == ROUND_CONCAT) continue;
+            if (c > 0) {
+                RoundList::Group& G = out.groups[c - 1];
+                G.cols = std::max(G.cols, layout_columns(*op));
+                G.rout = std::max(G.rout, op->rout);
+                continue;
+            }
+            // General kernel: the core and the rotations of an op live in shared
+            // memory when they fit the launch's size, otherwise in the
+            // (L1-cached) global work area; the size is the largest need of its
+            // non-dense ops (dense compressions with larger cores take the
+            // global path), so that more CTAs share an SM.
+            const bool dense = op->kind == ROUND_DENSE;
+            const long long k = op_columns(*op);
+            const long long ku = op->kind == ROUND_ORTHO ? op->r1 : std::min<long long>(op->m, k);
+            const long long kv = dense ? op->n : std::min<long long>(op->n, k);
             const long long need = ku * kv + kv * kv;
             if (!dense || need <= 3072) need_max = std::max(need_max, need);
         }
-    out.smem = std::min<long long>(need_max, fp32 ? kSmemBytesF32 / 4 : kSmemBytes / 8);
-    for (int g = 0; g < 2; ++g) {
-        RoundList::Group& G = out.groups[g];
-        G.warps = 8 >> g;
-        G.first = (int)index.size() - base;
-        take([&](int need) { return need == G.warps; });
-        G.count = (int)index.size() - base - G.first;
-        G.cols = G.rout = 1;
-        for (int i = G.first; i < G.first + G.count; ++i)
-            for (int o = begin[index[base + i]]; o < begin[index[base + i] + 1]; ++o) {
-                if (ops[o].kind == ROUND_SET || ops[o].kind == ROUND_CONCAT) continue;
-                G.cols = std::max(G.cols, layout_columns(ops[o]));
-                G.rout = std::max(G.rout, ops[o].rout);
-            }
     }
-}
+    // The worker list, appended to `index` in the given order.
+    void finish(const std::vector<int>& order, std::vector<int>& index) {
+        out.smem = std::min<long long>(need_max, fp32 ? kSmemBytesF32 / 4 : kSmemBytes / 8);
+        out.nw_general = count[0];
+        for (int g = 0; g < 2; ++g) {
+            out.groups[g].first = count[0] + (g == 1 ? count[1] : 0);
+            out.groups[g].count = count[1 + g];
+        }
+        out.workers = (int)index.size();
+        index.resize(index.size() + order.size());
+        int* at[3];
+        at[0] = index.data() + out.workers;
+        at[1] = at[0] + count[0];
+        at[2] = at[1] + count[1];
+        for (int w : order) *at[kernel[w]]++ = w;
+    }
+};
 
 }  // namespace
 
 void upload_round_list(Context& ctx, const std::vector<RoundOp>& ops,
-                       const std::vector<int>& begin, RoundList& out) {
+                       const std::vector<int>& begin, RoundList& out, int precision) {
     out.nw = 0;
     if (ops.empty() || begin.size() < 2) return;
-    for (const RoundOp& op : ops)
-        HMB_REQUIRE(op.kind == ROUND_SET || op.kind == ROUND_CONCAT || op_columns(op) <= kMaxK,
-                    HM_ERR_UNSUPPORTED, "low-rank rounding of more than 128 stacked columns");
-    out.nw = (int)begin.size() - 1;
-    out.ops.upload(ops, ctx.stream);
-    // the longest operation lists first, so that the last CTAs to start are
-    // short ones
-    std::vector<double> cost(out.nw, 0.0);
-    std::vector<int> order(out.nw), index(begin);
-    for (int w = 0; w < out.nw; ++w) {
-        order[w] = w;
-        for (int i = begin[w]; i < begin[w + 1]; ++i) cost[w] += op_cost(ops[i]);
+    const int nw = (int)begin.size() - 1;
+    Scheduler part[2] = {{false, out.sched[0], (size_t)nw}, {true, out.sched[1], (size_t)nw}};
+    std::vector<double> cost(nw, 0.0);
+    for (int w = 0; w < nw; ++w) {
+        const RoundOp *b = ops.data() + begin[w], *e = ops.data() + begin[w + 1];
+        for (const RoundOp* op = b; op < e; ++op) {
+            HMB_REQUIRE(op->kind == ROUND_SET || op->kind == ROUND_CONCAT || op_columns(*op) <= kMaxK,
+                        HM_ERR_UNSUPPORTED, "low-rank rounding of more than 128 stacked columns");
+            cost[w] += op_cost(*op);
+        }
+        for (int p = 0; p < 2; ++p)
+            if (precision < 0 || precision == p) part[p].add(b, e);
     }
-    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cost[a] > cost[b]; });
-    for (int fp32 = 0; fp32 < 2; ++fp32) schedule(ops, begin, order, fp32 != 0, index, out.sched[fp32]);
+    out.nw = nw;
+    out.ops.upload(ops, ctx.stream);
+    const std::vector<int> order = longest_first(cost);
+    std::vector<int> index;
+    index.reserve(begin.size() + 2 * (size_t)nw);
+    index = begin;
+    for (int p = 0; p < 2; ++p)
+        if (precision < 0 || precision == p) part[p].finish(order, index);
     out.index.upload(index, ctx.stream);
 }
 
@@ -893,7 +947,7 @@ void launch_round_list(Context& ctx, const RoundList& L, const RelocBases& bases
 void launch_round_workers(Context& ctx, const std::vector<RoundOp>& ops,
                           const std::vector<int>& begin, const char* name) {
     RoundList L;
-    upload_round_list(ctx, ops, begin, L);
+    upload_round_list(ctx, ops, begin, L, ctx.low_precision ? 1 : 0);
     launch_round_list(ctx, L, RelocBases{}, name);
 }
 

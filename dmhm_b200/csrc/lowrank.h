@@ -61,8 +61,9 @@ struct RoundList {
         Group groups[2];
     } sched[2];
 };
+// precision: 0 FP64 only, 1 FP32 only, -1 both (a list that is kept).
 void upload_round_list(Context& ctx, const std::vector<RoundOp>& ops,
-                       const std::vector<int>& begin, RoundList& out);
+                       const std::vector<int>& begin, RoundList& out, int precision = -1);
 void launch_round_list(Context& ctx, const RoundList& L, const RelocBases& bases,
                        const char* name);
 
