@@ -527,14 +527,14 @@ struct SymPlan {
 };
 
 struct SymKey {
-    const Structure* S = nullptr;
+    std::shared_ptr<const Structure> S;   // (kept: a matrix made anew on this grid shares it)
     int fresh = 1, maxRankC = 0, oversample = 0, maxA = 0, maxB = 0;
     double alpha = 0, beta = 0;
     std::vector<int> ra, rb, rc;
     std::vector<int> roots;   // flattened (a, b, c) sub-tree roots; empty: the whole matrix
     uint64_t hash = 0;
     bool operator==(const SymKey& o) const {
-        return hash == o.hash && S == o.S && fresh == o.fresh && maxRankC == o.maxRankC &&
+        return hash == o.hash && S->id == o.S->id && fresh == o.fresh && maxRankC == o.maxRankC &&
                oversample == o.oversample && maxA == o.maxA && maxB == o.maxB &&
                alpha == o.alpha && beta == o.beta && ra == o.ra && rb == o.rb && rc == o.rc &&
                roots == o.roots;
@@ -643,7 +643,7 @@ std::shared_ptr<SymPlan> get_plan(Context& ctx, const HMatrix& A, const HMatrix&
                                   const HMatrix& C, double alpha, double beta, bool fresh,
                                   int maxRankC, const std::vector<HHRoot>& roots) {
     SymKey key;
-    key.S = A.S.get();
+    key.S = A.S;
     key.fresh = fresh ? 1 : 0;
     key.maxRankC = maxRankC;
     key.oversample = ctx.oversample;
@@ -660,7 +660,7 @@ std::shared_ptr<SymPlan> get_plan(Context& ctx, const HMatrix& A, const HMatrix&
         key.roots.push_back(r.c);
     }
     uint64_t h = 1469598103934665603ULL;
-    h = fnv(h, &key.S, sizeof(key.S));
+    h = fnv(h, &A.S->id, sizeof(A.S->id));
     h = fnv(h, &key.fresh, sizeof(int) * 5);
     h = fnv(h, &key.alpha, sizeof(double) * 2);
     h = fnv(h, key.ra.data(), key.ra.size() * sizeof(int));

@@ -1422,14 +1422,14 @@ LayoutGroup& layout_group(Context& ctx, const HMatrix& H) {
         const unsigned char* c = static_cast<const unsigned char*>(p);
         for (size_t i = 0; i < n; ++i) h = (h ^ c[i]) * 1099511628211ULL;
     };
-    const Structure* S = H.S.get();
-    mix(&S, sizeof(S));
+    const uint64_t id = H.S->id;
+    mix(&id, sizeof(id));
     mix(&H.max_rank, sizeof(int));
     mix(H.rank.data(), H.rank.size() * sizeof(int));
     auto& L = ctx.layouts;
     for (size_t i = 0; i < L.size(); ++i) {
         LayoutGroup& g = *L[i];
-        if (g.hash == h && g.S == S && g.max_rank == H.max_rank && g.rank == H.rank) {
+        if (g.hash == h && g.S->id == id && g.max_rank == H.max_rank && g.rank == H.rank) {
             auto keep = L[i];
             L.erase(L.begin() + (long long)i);
             L.push_back(keep);
@@ -1438,7 +1438,7 @@ LayoutGroup& layout_group(Context& ctx, const HMatrix& H) {
         }
     }
     auto g = std::make_shared<LayoutGroup>();
-    g->S = S;
+    g->S = H.S;
     g->max_rank = H.max_rank;
     g->rank = H.rank;
     g->hash = h;

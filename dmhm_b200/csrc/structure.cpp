@@ -2,6 +2,7 @@
 #include "structure.h"
 
 #include <algorithm>
+#include <atomic>
 #include <cstdlib>
 #include <functional>
 #include <map>
@@ -70,6 +71,11 @@ bool same_structure(const Structure& a, const Structure& b) {
     return a.dim == b.dim && a.num_levels == b.num_levels && a.strong == b.strong &&
            a.dof == b.dof &&
            a.sizes[0] == b.sizes[0] && a.sizes[1] == b.sizes[1] && a.sizes[2] == b.sizes[2];
+}
+
+uint64_t Structure::next_id() {
+    static std::atomic<uint64_t> last{0};
+    return ++last;
 }
 
 std::shared_ptr<Structure> build_structure(int dim, const int* sizes, int num_levels,

@@ -5,6 +5,7 @@
 // include/dmhm/hmat2d.hpp:288-341, src/HMat2d/HMat2d.cpp:797-809,
 // include/dmhm/hmat3d.hpp:455-535, src/HMat3d/HMat3d.cpp:852-875).
 #pragma once
+#include <cstdint>
 #include <memory>
 #include <vector>
 
@@ -44,6 +45,9 @@ struct Structure {
     // block sizes are in rows)
     int dof = 1;
     int N = 0;        // rows = dof * grid points
+    // Of no other structure of the process, also not of one that is gone (an
+    // address is given out again): what caches tell structures apart by.
+    const uint64_t id = next_id();
 
     std::vector<Box> boxes;     // box 0 = the whole grid
     std::vector<int> leaf_box;  // leaf cluster -> box id (hierarchical order)
@@ -57,6 +61,9 @@ struct Structure {
     int num_clusters() const { return (int)leaf_box.size(); }
     int child(int b, int t, int s) const { return blocks[b].first_child + s + q * t; }
     bool in_subtree(int b, int root) const;  // b == root or a descendant
+
+  private:
+    static uint64_t next_id();
 };
 
 // Builds the structure (shared by all H-matrices over the same grid and

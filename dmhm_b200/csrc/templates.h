@@ -103,7 +103,7 @@ struct JobTemplate {
 // Matrices of one context with the same structure, rank cap and ranks (so the
 // same storage layout) and the work lists of their products.
 struct LayoutGroup {
-    const Structure* S = nullptr;
+    std::shared_ptr<const Structure> S;   // (kept: a matrix made anew on this grid shares it)
     int max_rank = 0;
     std::vector<int> rank;
     uint64_t hash = 0;
