@@ -355,7 +355,7 @@ __device__ __noinline__ int phase_qr(const Cta<R, NW> C, const RoundOp& op, cons
                                                           : U.p1 + (long long)c * U.ld1,
                               op.kind == ROUND_DENSE ? op.alpha : U.s1, row0, rows, c < n);
         }
-        if (op.kind == ROUND_DENSE && op.beta != 0.0) {
+        if (op.kind == ROUND_DENSE && op.beta != 0.0 && sizeof(R) == 8) {
             for (int l = 0; l < op.r2; ++l) {
                 Fetch<R, RPW> f;
                 f.get(op.u2 + (long long)l * op.ldu2, op.beta, row0, rows, lane);
@@ -369,6 +369,36 @@ __device__ __noinline__ int phase_qr(const Cta<R, NW> C, const RoundOp& op, cons
                 slab_axpy<R, CPL, RPW>(C.us(l & 1), a, w);
             }
             __syncwarp();
+        } else if (op.kind == ROUND_DENSE && op.beta != 0.0) {
+            // FP32: the two parts may cancel, so their sum is taken in FP64; kept
+            // behind the reflectors (work holds rows x n doubles) for V_out
+            R* sum = refl + (long long)rows * n;
+#pragma unroll
+            for (int s = 0; s < CPL; ++s) {
+                const int c = min(lane + 32 * s, n - 1);
+#pragma unroll
+                for (int i = 0; i < RPW; i += 4) {
+                    double t[4];
+                    const double* u[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int row = min(row0 + i + q, rows - 1);
+                        t[q] = op.alpha * op.u1[row + (long long)c * op.ldu1];
+                        u[q] = op.u2 + row;
+                    }
+                    for (int l = 0; l < op.r2; ++l) {
+                        const double v = op.beta * op.v2[c + (long long)l * op.ldv2];
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) t[q] = fma(u[q][(long long)l * op.ldu2], v, t[q]);
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const bool live = lane + 32 * s < n && row0 + i + q < rows;
+                        a[s][i + q] = live ? (R)t[q] : R(0);
+                        if (live) sum[row0 + i + q + (long long)c * rows] = (R)t[q];
+                    }
+                }
+            }
         }
     }
     // T is scaled by a power of two so that its largest entry lies in [1, 2):
@@ -826,27 +856,17 @@ __device__ __noinline__ void phase_u(const Cta<R, NW> C, const RoundOp& op, cons
     }
     __syncthreads();   // mat and the buffers are rewritten
     // inner products of `count` columns with U_out, kChunk per barrier;
-    // done(p, c, value) runs once per product
-    auto products = [&](int count, auto column, auto finish) {
+    // fetch(p, f) brings column p, finish(p, c, value) runs once per product
+    auto products = [&](int count, auto fetch, auto finish) {
         Fetch<R, RPW> f;
-        if (count > 0) {
-            const double* cp;
-            double sc;
-            column(0, cp, sc);
-            f.get(cp, sc, row0, rows, lane);
-        }
+        if (count > 0) fetch(0, f);
         for (int p0 = 0; p0 < count; p0 += kChunk) {
             const int buf = (p0 / kChunk) & 1, nc = min(kChunk, count - p0);
             R* ch = C.chunk(buf);
             for (int q = 0; q < nc; ++q) {
                 R* us = C.us(q & 1);
                 f.put(us, lane);
-                if (p0 + q + 1 < count) {
-                    const double* cp;
-                    double sc;
-                    column(p0 + q + 1, cp, sc);
-                    f.get(cp, sc, row0, rows, lane);
-                }
+                if (p0 + q + 1 < count) fetch(p0 + q + 1, f);
                 R s[CPL];
                 slab_dots<R, CPL, RPW>(us, a, s);
 #pragma unroll
@@ -864,14 +884,25 @@ __device__ __noinline__ void phase_u(const Cta<R, NW> C, const RoundOp& op, cons
         __syncthreads();
     };
     if (op.kind != ROUND_DENSE) {
-        products(U.cols(), [&](int p, const double*& cp, double& sc) { cp = U.col(p); sc = U.scale(p); },
+        products(U.cols(), [&](int p, Fetch<R, RPW>& f) { f.get(U.col(p), U.scale(p), row0, rows, lane); },
                  [&](int p, int c, R t) { mat[p * ld + c] = t; });
         return;
     }
     const int r2 = op.beta != 0.0 ? op.r2 : 0;
-    products(r2, [&](int p, const double*& cp, double& sc) { cp = op.u2 + (long long)p * op.ldu2; sc = op.beta; },
+    if (sizeof(R) == 4 && r2 > 0) {
+        const R* sum = refl + (long long)rows * n;   // alpha D + beta U2 V2^T (phase_qr)
+        products(n,
+                 [&](int p, Fetch<R, RPW>& f) {
+                     const R* col = sum + (long long)p * rows + row0;
+                     f.v0 = lane < RPW && row0 + lane < rows ? col[lane] : R(0);
+                     if (RPW > 32) f.v1 = 32 + lane < RPW && row0 + 32 + lane < rows ? col[32 + lane] : R(0);
+                 },
+                 [&](int p, int c, R t) { vo[p + (long long)c * n] = (double)t; });
+        return;
+    }
+    products(r2, [&](int p, Fetch<R, RPW>& f) { f.get(op.u2 + (long long)p * op.ldu2, op.beta, row0, rows, lane); },
              [&](int p, int c, R t) { mat[p * ld + c] = t; });
-    products(n, [&](int p, const double*& cp, double& sc) { cp = op.u1 + (long long)p * op.ldu1; sc = op.alpha; },
+    products(n, [&](int p, Fetch<R, RPW>& f) { f.get(op.u1 + (long long)p * op.ldu1, op.alpha, row0, rows, lane); },
              [&](int p, int c, R t) {
                  for (int l = 0; l < r2; ++l) t = r_fma((R)op.v2[p + (long long)l * op.ldv2], mat[l * ld + c], t);
                  vo[p + (long long)c * n] = (double)t;
@@ -1016,7 +1047,17 @@ __device__ void round_in_registers(const RoundOp& op, const Cta<R, NW> C, R tiny
 #define CALL(c, r) phase_u<R, NW, c, r>(C, op, U, nt, refl, k1, cols, tiny, uo, vo)
         HMB_SLABS(rout, U.rows, NW, CALL);
 #undef CALL
-        if (!dense) {
+        if (ortho && sizeof(R) == 4) {
+            // FP32: the orthonormal factor stays as it is, its combinations in FP64
+            const R* mat = C.mat();
+            for (int c = C.warp; c < rout; c += NW)
+                for (int i = C.lane; i < V.rows; i += 32) {
+                    double t = 0.0;
+                    for (int p = 0; p < k; ++p)
+                        t = fma(V.p1[i + (long long)p * V.ld1], (double)mat[p * C.L.ld + c], t);
+                    vo[i + (long long)c * V.rows] = t;
+                }
+        } else if (!dense) {
 #define CALL(c, r) phase_v<R, NW, c, r>(C, V, rout, vo)
             HMB_SLABS(rout, V.rows, NW, CALL);
 #undef CALL

@@ -83,3 +83,45 @@ def test_dense_compression_onto_a_rank_above_the_block(rank, low_precision):
     X = D.HMat2d(ctx=c).CopyFrom(A)
     A.Multiply(0.5, B, -0.7, X)
     assert relerr(X.Multiply(1.0, P), 0.5 * (a @ (b @ P)) - 0.7 * (a @ P)) < tol
+
+
+@pytest.mark.parametrize("low_precision", [False, True])
+def test_dense_compression_that_cancels(low_precision):
+    """C + A B where a low-rank block of C nearly cancels the dense x dense
+    product added to it: the sum is formed in FP64 before it is rounded, also by
+    the FP32 roundings, so what is left (1e-4 of the parts) keeps the
+    precision's own error: 1e-5 in FP32 (couplings of 1e-6), 1e-15 / 1e-4 and a
+    factor 100 for the sums in FP64."""
+    rng = np.random.default_rng(5)
+    t, k, s = (2, 0), (1, 0), (0, 0)
+    a, b = rng.standard_normal((16, 16)), rng.standard_normal((16, 16))
+    rest = 1e-4 * rng.standard_normal((16, 16))
+    c = D.Context(0)
+    c.set_low_precision(low_precision)
+    A = D.HMat2d.Unpack(pack(16, {(t, k): a}, {}), ctx=c)
+    B = D.HMat2d.Unpack(pack(16, {(k, s): b}, {}), ctx=c)
+    X = D.HMat2d.Unpack(pack(16, {}, {(t, s): (rest - 0.5 * a @ b, np.eye(16))}), ctx=c)
+    A.Multiply(0.5, B, 1.0, X)
+    got = X.Multiply(1.0, np.eye(SIDE * SIDE))
+    at = {q: o for q, o, _ in boxes(LEVELS - 1)}
+    assert relerr(got[at[t]:at[t] + 16, at[s]:at[s] + 16], rest) < (1e-5 if low_precision else 1e-9)
+
+
+@pytest.mark.parametrize("low_precision", [False, True])
+@pytest.mark.parametrize("rank", [4, 16, 31])
+def test_sampled_products_of_a_small_matrix(rank, low_precision):
+    """One low-rank approximation of a product of 256 points (the orthonormal
+    form of the register roundings, 8 warps): exact where the product's rank is
+    the sample's."""
+    rng = np.random.default_rng(rank)
+    U, V = rng.standard_normal((16, rank)), rng.standard_normal((16, rank))
+    dense = {((1, 1), (2, 1)): U @ V.T}
+    b = {((2, 1), (q, 2)): rng.standard_normal((16, 16)) for q in (1, 2, 3)}
+    c = D.Context(0)
+    c.set_oversample(1)
+    c.set_low_precision(low_precision)
+    A, B = (D.HMat2d.Unpack(pack(rank, d, {}), ctx=c) for d in (dense, b))
+    got_u, got_v = A.LowRankProduct(1.5, B)
+    P = rng.standard_normal((SIDE * SIDE, 3))
+    assert relerr(got_u @ (got_v.T @ P), 1.5 * full(dense, {}) @ (full(b, {}) @ P)) < (
+        1e-5 if low_precision else 1e-12)
