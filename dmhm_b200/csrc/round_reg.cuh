@@ -209,15 +209,8 @@ __device__ __forceinline__ void sum_slabs(const Cta<R, NW>& C, int buf, R (&s)[C
     }
 }
 
-// 1 / x to rounding by Newton's iteration from the hardware's approximation
-// (x normal): half the latency of the division, which every step waits for.
-__device__ __forceinline__ double reciprocal(double x) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    y = fma(y, fma(-x, y, 1.0), y);
-    y = fma(y, fma(-x, y, 1.0), y);
-    return fma(y, fma(-x, y, 1.0), y);
-}
+// (FP64: a call-free form of 1 / x; every step waits for it)
+__device__ __forceinline__ double reciprocal(double x) { return __drcp_rn(x); }
 __device__ __forceinline__ float reciprocal(float x) { return 1.0f / x; }
 
 // One elimination step: the reflector of column p on row j (the first row of
