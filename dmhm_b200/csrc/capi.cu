@@ -378,8 +378,7 @@ int hm_fp64_split_choice(hm_matrix h, const double* B, int ldb, int nrhs, int* w
         HMB_REQUIRE(h->h.S != nullptr, HM_ERR_ARGUMENT, "empty H-matrix");
         HMB_REQUIRE(nrhs > 0 && ldb >= std::max(1, h->h.width()), HM_ERR_ARGUMENT,
                     "bad right-hand sides");
-        // the whole product, as hm_multiply_dense runs it (a tuning run
-        // writes into scratch, so no output is needed)
+        // the whole product, as hm_multiply_dense runs it
         MatJob J{&h->h, 0, false, 1.0, 0.0, B, ldb, nullptr, std::max(1, h->h.height()), nrhs};
         *which = fp64_split_for(*h->h.ctx, {J});
     });

@@ -227,13 +227,12 @@ HM_API int hm_set_tf32_kernel(hm_context ctx, int which);
 HM_API int hm_tf32_kernel_choice(hm_matrix h, const double* B, int ldb, int nrhs, int* which);
 /*
  * FP64 products of 9 to 16 columns (hm_multiply_dense and the H*H sampling
- * products) run either as one pass of the FP64 tensor-core 64 x 64 tiles (1)
- * or as passes of at most 8 columns (2); which
- * is faster depends on the operator.  hm_set_fp64_split(ctx, 0) (the
- * default) times both the first time a (layout, job count, column count)
- * occurs and keeps the faster; hm_fp64_split_choice reports (and if need be
- * tunes) the form hm_multiply_dense uses for nrhs columns (DEVICE B).  No
- * counterpart in the reference (it calls one BLAS routine per block).
+ * products) run as one pass of the FP64 tensor-core tiles of 16 columns (1)
+ * or as passes of at most 8 columns (2).  hm_set_fp64_split(ctx, 0) (the
+ * default) takes the single pass, which reads every block once and is the
+ * faster one wherever both were measured; hm_fp64_split_choice reports the
+ * form hm_multiply_dense uses for nrhs columns (DEVICE B).  No counterpart in
+ * the reference (it calls one BLAS routine per block).
  */
 HM_API int hm_set_fp64_split(hm_context ctx, int which);
 HM_API int hm_fp64_split_choice(hm_matrix h, const double* B, int ldb, int nrhs, int* which);
