@@ -9,6 +9,7 @@
 
 #include <algorithm>
 
+#include "fp64_tiles.cuh"
 #include "kernel_limits.h"
 
 namespace hmb {
@@ -23,31 +24,6 @@ constexpr size_t kSmem = 2ull * kStages * kStage * sizeof(double);
 
 __device__ __forceinline__ double ld_op(const double* X, int ld, bool trans, int i, int j) {
     return trans ? X[j + (long long)i * ld] : X[i + (long long)j * ld];
-}
-
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-__device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-                 : "+d"(d[0]), "+d"(d[1])
-                 : "d"(a), "d"(b));
-}
-
-// Two doubles (`bytes` of them valid, zeros beyond) to the shared address d;
-// `any` is a valid, 16-byte aligned address for copies of nothing.
-__device__ __forceinline__ void copy_pair(unsigned d, const double* src, int bytes, bool aligned,
-                                          const double* any) {
-    if (aligned) {
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(bytes ? src : any),
-                     "r"(bytes));
-    } else {
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(bytes ? src : any),
-                     "r"(bytes ? 8 : 0));
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d + 8),
-                     "l"(bytes > 8 ? src + 1 : any), "r"(bytes > 8 ? 8 : 0));
-    }
 }
 
 // Stages 16 inner indices of one operand: `wide` (at most 64) rows of op(A) or

@@ -25,6 +25,7 @@
 #include <map>
 
 #include "engine.h"
+#include "fp64_tiles.cuh"
 #include "kernel_limits.h"
 #include "templates.h"
 
@@ -112,20 +113,19 @@ __device__ __forceinline__ long long piece_slot(long long q, long long wa, bool 
     return 2 * q + ((q == wa && !wa_starts_here) ? 1 : 0);
 }
 
-// Narrow: k <= NC.  Persistent warps stream their share of the items' rows.
-// A lane owns rows p and p + 32 of a 64-row step and loads JC = 16/NC columns
-// of W for both (2 JC loads in flight); the 16 partial sums of a column chunk
+// One column.  Persistent warps stream their share of the items' rows.  A
+// lane owns rows p and p + 32 of a 64-row step and loads JC = 16 columns of W
+// for both (2 JC loads in flight); the 16 partial sums of a column chunk
 // are reduced across the warp by a transposing butterfly.
-template <int NC>
 __global__ void __launch_bounds__(kThreads, 2)
 p1_stream_kernel(const JobExec* __restrict__ jobs, int njobs, const JobExec job0, long long C,
                  long long GW, double* __restrict__ S, int rmax,
                  const int* __restrict__ start) {
-    constexpr int JC = 16 / NC;
+    constexpr int JC = 16;
     const int lane = threadIdx.x & 31;
     const long long w = (long long)blockIdx.x * kWarps + (threadIdx.x >> 5);
     if (w >= GW) return;
-    const long long slot_len = (long long)rmax * NC;
+    const long long slot_len = rmax;
     long long g = split_start(w, GW, C);
     const long long gend = split_start(w + 1, GW, C);
     bool first = true;
@@ -148,11 +148,11 @@ p1_stream_kernel(const JobExec* __restrict__ jobs, int njobs, const JobExec job0
         }
         const P1T it = J.p1[item];
         if (item + 1 < J.n1) asm volatile("prefetch.global.L1 [%0];" ::"l"(J.p1 + item + 1));
-        const int K = J.k, ldin = J.ldin, r = it.r;
+        const int r = it.r;
         const int p0 = (int)(local - it.c0);
         const int p1 = (int)min((long long)it.nin, gend - J.p1_begin - it.c0);
         const bool whole = p0 == 0 && p1 == it.nin;
-        double* dst = whole ? J.T + it.t_rel * K : S + (2 * w + (first ? 0 : 1)) * slot_len;
+        double* dst = whole ? J.T + it.t_rel : S + (2 * w + (first ? 0 : 1)) * slot_len;
         const double* in = J.in + it.in_off;
         for (int j0 = 0; j0 < r; j0 += JC) {
             double v[16];
@@ -162,28 +162,21 @@ p1_stream_kernel(const JobExec* __restrict__ jobs, int njobs, const JobExec job0
             for (int pa = p0 + lane; pa < p1; pa += 64) {
                 const int pb = pa + 32;
                 const bool okb = pb < p1;
-                double wa[JC], wb[JC], xa[NC], xb[NC];
+                double wa[JC], wb[JC];
 #pragma unroll
                 for (int jj = 0; jj < JC; ++jj) {
                     const bool cj = j0 + jj < r;
                     wa[jj] = cj ? __ldg(wp + pa + (long long)jj * it.ldw) : 0.0;
                     wb[jj] = (okb && cj) ? __ldg(wp + pb + (long long)jj * it.ldw) : 0.0;
                 }
+                const double xa = __ldg(in + pa), xb = okb ? __ldg(in + pb) : 0.0;
 #pragma unroll
-                for (int c = 0; c < NC; ++c) {
-                    xa[c] = (c < K) ? __ldg(in + pa + (long long)c * ldin) : 0.0;
-                    xb[c] = (okb && c < K) ? __ldg(in + pb + (long long)c * ldin) : 0.0;
-                }
-#pragma unroll
-                for (int jj = 0; jj < JC; ++jj)
-#pragma unroll
-                    for (int c = 0; c < NC; ++c)
-                        v[jj * NC + c] = fma(wb[jj], xb[c], fma(wa[jj], xa[c], v[jj * NC + c]));
+                for (int jj = 0; jj < JC; ++jj) v[jj] = fma(wb[jj], xb, fma(wa[jj], xa, v[jj]));
             }
             warp_transpose_sum16(v, lane);
             if ((lane & 1) == 0) {
-                const int f = lane >> 1, jj = f / NC, c = f % NC;
-                if (j0 + jj < r && c < K) dst[(j0 + jj) + (long long)c * r] = v[0];
+                const int f = lane >> 1;
+                if (j0 + f < r) dst[j0 + f] = v[0];
             }
         }
         if (!whole) {
@@ -197,8 +190,8 @@ p1_stream_kernel(const JobExec* __restrict__ jobs, int njobs, const JobExec job0
             if (last) {
                 __threadfence();
                 const bool wa_here = split_start(wa, GW, C) == G0;
-                double* T = J.T + it.t_rel * K;
-                for (int o = lane; o < r * K; o += 32) {
+                double* T = J.T + it.t_rel;
+                for (int o = lane; o < r; o += 32) {
                     double t = 0.0;
                     for (long long q = wa; q <= wb; ++q)
                         t += __ldcg(S + piece_slot(q, wa, wa_here) * slot_len + o);
@@ -220,13 +213,6 @@ __device__ __forceinline__ double load_a(const double* hb, const P2Entry& e, int
     return e.transA ? __ldg(A + p + (long long)i * e.lda) : __ldg(A + i + (long long)p * e.lda);
 }
 
-// B operand of an entry: (pointer to element (0,0), leading dimension).
-__device__ __forceinline__ void entry_b(const P2Entry& e, const JobExec& J, const double*& B,
-                                       int& ldb) {
-    if (e.b_from_t) { B = J.T + e.b_off * J.k; ldb = e.ldt; }
-    else { B = J.in + e.b_off; ldb = J.ldin; }
-}
-
 __device__ __forceinline__ void store_out(const JobExec& J, const P2T& it, int i, int c,
                                           double v) {
     double* y = J.out + it.out_off + (it.r0 + i) + (long long)c * J.ldout;
@@ -234,20 +220,19 @@ __device__ __forceinline__ void store_out(const JobExec& J, const P2T& it, int i
     *y = J.beta == 0.0 ? al * v : al * v + J.beta * *y;
 }
 
-// Narrow: columns <= NC, rows <= 32, a streaming (HBM-bound) kernel.
+// One column, tiles of at most 32 rows, a streaming (HBM-bound) kernel.
 // Persistent warps stream their share of the tiles' concatenated inner
 // dimensions (entry e of a tile covers [cbeg, cbeg + inner)).  Within a
 // warp, "column workers" (sub-groups of lanes, one lane per row) split the
 // piece evenly and keep U columns of loads in flight.
-template <int NC>
 __global__ void __launch_bounds__(kThreads, 2)
 p2_stream_kernel(const JobExec* __restrict__ jobs, int njobs, const JobExec job0, long long C,
                  long long GW, double* __restrict__ S, const int2* __restrict__ start) {
-    constexpr int U = NC == 1 ? 16 : 4;
+    constexpr int U = 16;
     const int lane = threadIdx.x & 31;
     const long long w = (long long)blockIdx.x * kWarps + (threadIdx.x >> 5);
     if (w >= GW) return;
-    constexpr long long slot_len = 32LL * NC;
+    constexpr long long slot_len = 32;
     long long g = split_start(w, GW, C);
     const long long gend = split_start(w + 1, GW, C);
     bool first = true;
@@ -279,7 +264,6 @@ p2_stream_kernel(const JobExec* __restrict__ jobs, int njobs, const JobExec job0
             }
             it = J.p2[tile];
         }
-        const int cols = J.k;
         const int q0 = (int)(local - it.c0);
         const int q1 = (int)min((long long)it.width, gend - J.p2_begin - it.c0);
         const bool whole = q0 == 0 && q1 == it.width;
@@ -289,9 +273,7 @@ p2_stream_kernel(const JobExec* __restrict__ jobs, int njobs, const JobExec job0
         const int sub = lane / RL, rl = lane % RL, nsub = 32 / RL;
         const bool row_ok = rl < it.rows;
         const int row = it.r0 + rl;
-        double acc[NC];
-#pragma unroll
-        for (int c = 0; c < NC; ++c) acc[c] = 0.0;
+        double acc = 0.0;
         {
             const int chunk = (q1 - q0 + nsub - 1) / nsub;
             int p = q0 + sub * chunk;
@@ -310,54 +292,35 @@ p2_stream_kernel(const JobExec* __restrict__ jobs, int njobs, const JobExec job0
             while (p < pend) {
                 const P2Entry e = J.ent[ei];
                 if (ei + 1 < it.e1) asm volatile("prefetch.global.L1 [%0];" ::"l"(J.ent + ei + 1));
-                const double* EB;
-                int ldb;
-                entry_b(e, J, EB, ldb);
+                const double* EB = e.b_from_t ? J.T + e.b_off : J.in + e.b_off;
                 const int stop = min(pend, e.cbeg + e.inner);
                 int q = p - e.cbeg;                 // column within the entry
                 const int qstop = stop - e.cbeg;
                 for (; q + U - 1 < qstop; q += U) {
-                    double av[U], bv[U][NC];
+                    double av[U], bv[U];
 #pragma unroll
                     for (int u = 0; u < U; ++u) {
-#pragma unroll
-                        for (int c = 0; c < NC; ++c)
-                            bv[u][c] = (c < cols) ? __ldg(EB + (q + u) + (long long)c * ldb) : 0.0;
+                        bv[u] = __ldg(EB + (q + u));
                         av[u] = row_ok ? load_a(J.hb, e, row, q + u) : 0.0;
                     }
 #pragma unroll
-                    for (int u = 0; u < U; ++u)
-#pragma unroll
-                        for (int c = 0; c < NC; ++c) acc[c] = fma(av[u], bv[u][c], acc[c]);
+                    for (int u = 0; u < U; ++u) acc = fma(av[u], bv[u], acc);
                 }
                 for (; q < qstop; ++q) {
                     const double av = row_ok ? load_a(J.hb, e, row, q) : 0.0;
-#pragma unroll
-                    for (int c = 0; c < NC; ++c)
-                        if (c < cols) acc[c] = fma(av, __ldg(EB + q + (long long)c * ldb), acc[c]);
+                    acc = fma(av, __ldg(EB + q), acc);
                 }
                 p = stop;
                 ++ei;
             }
         }
         // reduce over the column sub-groups (lanes with equal rl)
-#pragma unroll
-        for (int c = 0; c < NC; ++c) {
-            double v = acc[c];
-            for (int o = 16; o >= RL; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            acc[c] = v;
-        }
+        for (int o = 16; o >= RL; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
         if (whole) {
-            if (sub == 0 && row_ok)
-#pragma unroll
-                for (int c = 0; c < NC; ++c)
-                    if (c < cols) store_out(J, it, rl, c, acc[c]);
+            if (sub == 0 && row_ok) store_out(J, it, rl, 0, acc);
         } else {
-            double* P = S + (2 * w + (first ? 0 : 1)) * slot_len;   // 32 x NC, ld 32
-            if (sub == 0 && row_ok)
-#pragma unroll
-                for (int c = 0; c < NC; ++c)
-                    if (c < cols) P[rl + 32 * c] = acc[c];
+            double* P = S + (2 * w + (first ? 0 : 1)) * slot_len;
+            if (sub == 0 && row_ok) P[rl] = acc;
             __threadfence();
             __syncwarp();
             const long long G0 = J.p2_begin + it.c0;
@@ -368,12 +331,11 @@ p2_stream_kernel(const JobExec* __restrict__ jobs, int njobs, const JobExec job0
             if (last) {
                 __threadfence();
                 const bool wa_here = split_start(wa, GW, C) == G0;
-                for (int o = lane; o < it.rows * cols; o += 32) {
-                    const int i = o % it.rows, c = o / it.rows;
+                for (int i = lane; i < it.rows; i += 32) {
                     double t = 0.0;
                     for (long long q = wa; q <= wb; ++q)
-                        t += __ldcg(S + piece_slot(q, wa, wa_here) * slot_len + i + 32 * c);
-                    store_out(J, it, i, c, t);
+                        t += __ldcg(S + piece_slot(q, wa, wa_here) * slot_len + i);
+                    store_out(J, it, i, 0, t);
                 }
                 if (lane == 0) J.cnt2[tile] = 0;
             }
@@ -456,16 +418,6 @@ __device__ __forceinline__ float round_tf32(double x) {
     uint32_t r;
     asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"((float)x));
     return __uint_as_float(r);
-}
-
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-__device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-                 : "+d"(d[0]), "+d"(d[1])
-                 : "d"(a), "d"(b));
 }
 
 // TF32 tiles: slot s = ((mb * 4 + nb) * 4 + e) of MMA block (mb, nb) (16 x 8)
@@ -809,20 +761,6 @@ struct Tile64 {
     static constexpr size_t smem = (size_t)STAGES * (ASZ + BSZ) * sizeof(double);
 };
 
-// Two doubles src[0], src[1] (`bytes` of them valid, zeros beyond) to the
-// shared address d; `any` is a valid address for copies of nothing.
-__device__ __forceinline__ void copy_pair(unsigned d, const double* src, int bytes, bool aligned,
-                                          const double* any) {
-    if (aligned) {
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(bytes ? src : any),
-                     "r"(bytes));
-    } else {
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(bytes ? src : any),
-                     "r"(bytes ? 8 : 0));
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d + 8),
-                     "l"(bytes > 8 ? src + 1 : any), "r"(bytes > 8 ? 8 : 0));
-    }
-}
 __device__ __forceinline__ bool even16(const double* p, long long stride) {
     return ((reinterpret_cast<size_t>(p) | (size_t)(stride << 3)) & 15) == 0;
 }
@@ -1092,7 +1030,7 @@ wide64_kernel(const JobExec* __restrict__ jobs, int njobs, const JobExec job0, l
                     for (int m = 0; m < MG; ++m)
 #pragma unroll
                         for (int c = 0; c < NB; ++c) v[m][c][0] = v[m][c][1] = 0.0;
-#pragma unroll(NT == 16 ? 2 : 4)
+#pragma unroll(NT == 16 ? (ONE ? 2 : 1) : 4)
                     for (long long w = wa; w <= wb; ++w) {
                         const double2* p =
                             part + piece_slot(w, wa, wa_here) * (WT * NT / 2) + m0 * NB * WTHREADS;
@@ -1507,31 +1445,30 @@ const int2* warp_starts2(Context& ctx, JobTemplate& T, long long GW) {
     return d.get();
 }
 
-template <int NC>
 void launch_narrow(Context& ctx, const JobExec* jobs_d, int nj, const JobExec& job0,
                    long long c1, long long c2, int rmax, JobTemplate* single) {
     cudaStream_t st = ctx.stream;
     if (c1 > 0) {
         const long long g = std::min<long long>(ceil_div(c1, kWarps),
-                                                persistent_grid(ctx, p1_stream_kernel<NC>, kThreads));
+                                                persistent_grid(ctx, p1_stream_kernel, kThreads));
         const long long GW = std::min<long long>(g * kWarps, c1);
         const int* starts = single ? warp_starts1(ctx, *single, GW) : nullptr;
         DeviceBuffer<double> S;
-        S.allocate((size_t)(2 * GW * rmax * NC), st);
+        S.allocate((size_t)(2 * GW * rmax), st);
         LaunchScope ls(ctx, "hmm_lowrank_inner");
-        p1_stream_kernel<NC><<<(unsigned)g, kThreads, 0, st>>>(jobs_d, nj, job0, c1, GW, S.get(),
+        p1_stream_kernel<<<(unsigned)g, kThreads, 0, st>>>(jobs_d, nj, job0, c1, GW, S.get(),
                                                                rmax, starts);
         HMB_CHECK_LAUNCH();
     }
     if (c2 > 0) {
         const long long g = std::min<long long>(ceil_div(c2, kWarps),
-                                                persistent_grid(ctx, p2_stream_kernel<NC>, kThreads));
+                                                persistent_grid(ctx, p2_stream_kernel, kThreads));
         const long long GW = std::min<long long>(g * kWarps, c2);
         const int2* starts = single ? warp_starts2(ctx, *single, GW) : nullptr;
         DeviceBuffer<double> S;
-        S.allocate((size_t)(2 * GW * 32 * NC), st);
+        S.allocate((size_t)(2 * GW * 32), st);
         LaunchScope ls(ctx, "hmm_row_tiles");
-        p2_stream_kernel<NC><<<(unsigned)g, kThreads, 0, st>>>(jobs_d, nj, job0, c2, GW, S.get(),
+        p2_stream_kernel<<<(unsigned)g, kThreads, 0, st>>>(jobs_d, nj, job0, c2, GW, S.get(),
                                                                starts);
         HMB_CHECK_LAUNCH();
     }
@@ -1902,7 +1839,7 @@ void run_jobs_direct(Context& ctx, const std::vector<MatJob>& jobs, bool tf32) {
     const int nj = (int)ex.size();
     if (!wide) {
         JobTemplate* single = nj == 1 ? tmpl[first_job].get() : nullptr;
-        launch_narrow<1>(ctx, jobs_d, nj, job0, n1, n2, rmax, single);
+        launch_narrow(ctx, jobs_d, nj, job0, n1, n2, rmax, single);
         launch_zero_tiles(ctx, tmpl, jobs, jobs_d, job0);
         return;
     }

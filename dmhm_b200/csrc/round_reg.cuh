@@ -29,6 +29,7 @@
 // 924 -> 221 ms in 36; FP32, 72 x 68 grid, 765 -> 192 ms in 28.
 #pragma once
 
+#include "fp64_tiles.cuh"
 #include "round_sizing.h"
 
 namespace hmb {
@@ -520,12 +521,6 @@ __device__ __noinline__ void phase_lq(const Cta<R, NW> C, int k1, int n) {
     __syncthreads();
 }
 
-__device__ __forceinline__ void dmma884(double (&d)[2], double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-                 : "+d"(d[0]), "+d"(d[1])
-                 : "d"(a), "d"(b));
-}
-
 // Whether two of the n columns (rows of mat, each of `len` entries) are still
 // coupled above the threshold; squared norms to nrm.  The Gram matrix in 8 x 8
 // tiles on the FP64 tensor pipe, its diagonal first.
@@ -544,8 +539,8 @@ __device__ __forceinline__ bool coupled(const Cta<R, NW> C, int n, int len, R ti
             const double b0 = k + t < len ? (double)pb[k + t] : 0.0;
             const double a1 = k + 4 + t < len ? (double)pa[k + 4 + t] : 0.0;
             const double b1 = k + 4 + t < len ? (double)pb[k + 4 + t] : 0.0;
-            dmma884(d, a0, b0);
-            dmma884(e, a1, b1);
+            dmma(d, a0, b0);
+            dmma(e, a1, b1);
         }
         d[0] += e[0];
         d[1] += e[1];
