@@ -364,34 +364,64 @@ __device__ __noinline__ int phase_qr(const Cta<R, NW> C, const RoundOp& op, cons
             }
             __syncwarp();
         } else if (op.kind == ROUND_DENSE && op.beta != 0.0) {
-            // FP32: the two parts may cancel, so their sum is taken in FP64; kept
-            // behind the reflectors (work holds rows x n doubles) for V_out
+            // FP32: the two parts may cancel, so their sum is taken in FP64, some
+            // rows at a time; kept behind the reflectors (work holds rows x n
+            // doubles) for V_out
             R* sum = refl + (long long)rows * n;
+            constexpr int CH = RPW % 8 == 0 ? 8 : 4;
 #pragma unroll
-            for (int s = 0; s < CPL; ++s) {
-                const int c = min(lane + 32 * s, n - 1);
+            for (int i0 = 0; i0 < RPW; i0 += CH) {
+                double t[CPL][CH], v[CPL], u = 0.0;
+                const double* v2[CPL];
+                const bool fetches = lane < CH && row0 + i0 + lane < rows;
+                const double* u2 = op.u2 + row0 + i0 + lane;
 #pragma unroll
-                for (int i = 0; i < RPW; i += 4) {
-                    double t[4];
-                    const double* u[4];
+                for (int s = 0; s < CPL; ++s) {
+                    const int c = min(lane + 32 * s, n - 1);
+                    v2[s] = op.v2 + c;
+                    v[s] = op.r2 > 0 ? *v2[s] : 0.0;
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const int row = min(row0 + i + q, rows - 1);
-                        t[q] = op.alpha * op.u1[row + (long long)c * op.ldu1];
-                        u[q] = op.u2 + row;
-                    }
-                    for (int l = 0; l < op.r2; ++l) {
-                        const double v = op.beta * op.v2[c + (long long)l * op.ldv2];
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) t[q] = fma(u[q][(long long)l * op.ldu2], v, t[q]);
-                    }
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const bool live = lane + 32 * s < n && row0 + i + q < rows;
-                        a[s][i + q] = live ? (R)t[q] : R(0);
-                        if (live) sum[row0 + i + q + (long long)c * rows] = (R)t[q];
+                    for (int q = 0; q < CH; ++q) {
+                        const int row = row0 + i0 + q;
+                        t[s][q] = row < rows ? op.alpha * op.u1[row + (long long)c * op.ldu1] : 0.0;
                     }
                 }
+                if (fetches && op.r2 > 0) u = *u2;
+                for (int l = 0; l < op.r2; ++l) {
+                    double* us = reinterpret_cast<double*>(C.us(l & 1));
+                    if (lane < CH) us[lane] = u;
+                    __syncwarp();
+                    double w[CPL];
+#pragma unroll
+                    for (int s = 0; s < CPL; ++s) w[s] = op.beta * v[s];
+                    if (l + 1 < op.r2) {   // the next column of U2 and V2
+                        u2 += op.ldu2;
+                        if (fetches) u = *u2;
+#pragma unroll
+                        for (int s = 0; s < CPL; ++s) {
+                            v2[s] += op.ldv2;
+                            v[s] = *v2[s];
+                        }
+                    }
+#pragma unroll
+                    for (int q = 0; q < CH; q += 2) {
+                        const double2 x = *reinterpret_cast<const double2*>(us + q);
+#pragma unroll
+                        for (int s = 0; s < CPL; ++s) {
+                            t[s][q] = fma(x.x, w[s], t[s][q]);
+                            t[s][q + 1] = fma(x.y, w[s], t[s][q + 1]);
+                        }
+                    }
+                }
+                __syncwarp();
+#pragma unroll
+                for (int s = 0; s < CPL; ++s)
+#pragma unroll
+                    for (int q = 0; q < CH; ++q) {
+                        const int c = lane + 32 * s, row = row0 + i0 + q;
+                        a[s][i0 + q] = c < n && row < rows ? (R)t[s][q] : R(0);
+                        if (c < n && row < rows) sum[row + (long long)c * rows] = (R)t[s][q];
+                    }
             }
         }
     }
