@@ -789,10 +789,8 @@ __device__ __noinline__ int phase_jacobi(const Cta<R, NW> C, int k1, R tiny) {
         for (int i = C.lane; i < k1; i += 32)
             if (i < c || c >= k1) mat[c * ld + i] = R(0);
     __syncthreads();
-    // couplings left: the general kernel's level (one that grows with the
-    // columns' rounding, eps sqrt(k1), saves 5 % on complex 24 x 24, whose k1 is
-    // up to 72, and leaves couplings of up to 2e-15)
-    const R jt = sizeof(R) == 8 ? R(1e-15) : R(1e-6), jt2 = jt * jt;
+    const R eps = sizeof(R) == 8 ? R(2.220446049250313e-16) : R(1e-6);
+    const R jt2 = sizeof(R) == 8 ? eps * eps * R(max(k1, 20)) : eps * eps;
     for (int sweep = 0; sweep < kMaxSweeps && coupled<R, NW>(C, n, k1, tiny, jt2); ++sweep) {
         if (n <= 16) {
             if (C.warp == 0) jacobi_sweep<R, NW, 8, 4, 1>(C, n, k1, tiny, jt2);
