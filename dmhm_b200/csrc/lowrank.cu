@@ -753,11 +753,13 @@ void launch_round_reg(const RoundList& L, const int* workers, const RoundList::G
 }
 
 // The groups of a list are independent (each worker writes its own block)
-// and each leaves SMs idle at its end, so they run at the same time: those
-// with the longest CTAs first (the general kernel, then 8 warps), by the
-// priorities of the side streams.  Streams of one priority start in an order
-// that changes with the build: SchulzInvert mixed 72 x 68 took 330 ms or,
-// when the general kernel came last and ran on nearly alone, 378.
+// and each leaves SMs idle at its end, so they run at the same time, by the
+// priorities of the side streams the general kernel first (its CTAs are the
+// longest), then the 4-warp form, whose CTAs fit beside the others', then the
+// 8-warp one.  Streams of one priority start in an order that changes with the
+// build and with the streams made before: mixed SchulzInvert 72 x 68 took 330
+// ms or, when the general kernel came last and ran on nearly alone, 378; with
+// the 8-warp form second 330 or 353 (64 x 64 product 19.3 ms), so 328 (18.6).
 template <typename R>
 void launch_round_typed(Context& ctx, const RoundList& L, const RelocBases& bases,
                         const char* name) {
@@ -787,7 +789,8 @@ void launch_round_typed(Context& ctx, const RoundList& L, const RelocBases& base
             L.ops.get(), L.index.get(), workers, sch.smem, bases, numflag);
         HMB_CHECK_LAUNCH();
     }
-    for (const RoundList::Group& g : sch.groups) {
+    for (int i = 1; i >= 0; --i) {   // 4 warps, then 8
+        const RoundList::Group& g = sch.groups[i];
         if (g.count == 0) continue;
         const cudaStream_t st = stream();
         if (g.warps == 4) launch_round_reg<R, 4>(L, workers, g, bases, numflag, st);
