@@ -489,10 +489,11 @@ __device__ void do_round(const RoundOp& op, R* dyn, long long smem_elems, RoundS
 
     // ---- stacked factors ---------------------------------------------------
     if (op.kind == ROUND_GENERAL) {
-        // [beta U2, alpha U1], [V2, V1]: U2 (the block's current factors, the
-        // output of an earlier rounding) has orthogonal columns and V2
-        // orthonormal ones, so the leading part of the core is already
-        // diagonal and the Jacobi sweeps mostly rotate the new columns in
+        // [beta U2, alpha U1], [V2, V1]: the columns of the block's current
+        // factors U2 and V2, the output of an earlier rounding, are orthogonal
+        // (the scale in U2 from this kernel, in V2 from the register form), so
+        // the leading part of the core is already diagonal and the Jacobi
+        // sweeps mostly rotate the new columns in
         const int r2 = op.r2;
         for_each_entry(m, k, [&](int i, int c) {
             Ucat[i + (long long)c * m] =

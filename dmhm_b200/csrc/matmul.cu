@@ -9,13 +9,16 @@
 // input.  Each (H-matrix, root, op) has a template -- its work lists, built
 // once and kept on the device -- and a batch of jobs runs as two launches:
 //   phase 1: T_b = W_b^T X_b for every low-rank block b of every job
-//            (W = V, or U for the transpose): for one column one warp per
-//            row segment of a block, whole blocks per CTA; otherwise one
-//            CTA per block and 32-column tile;
+//            (W = V, or U for the transpose): for one column the blocks' rows
+//            shared out evenly among warps; otherwise tiles of 64 columns of
+//            the W's that share a source box, in chunks of 16 inner indices
+//            shared out evenly among persistent CTAs;
 //   phase 2: for every output row tile of every job, Y_tile = alpha * (sum
 //            over the dense leaves and low-rank blocks covering the tile of
-//            A_e(tile rows) * B_e) + beta * Y_tile, one CTA per tile, so each
-//            output element is written once (no atomics, deterministic).
+//            A_e(tile rows) * B_e) + beta * Y_tile, shared out likewise; a
+//            tile cut between warps or CTAs is added up in their order by the
+//            one that finishes last, so each output element is written once
+//            and the sums do not depend on the timing.
 // Every stored matrix entry is read exactly once per launch pair.  A CTA finds
 // its job by binary search over the jobs' first work-item indices.
 #include <algorithm>
@@ -729,7 +732,7 @@ wide_tf32_kernel(const JobExec* __restrict__ jobs, int njobs, const JobExec job0
 //
 // Bound by the FP64 tensor pipe from about 40 columns on, by HBM below.  The
 // operands of a chunk (16 inner indices) reach shared memory by 16-byte
-// cp.async three chunks ahead, in the order memory has them: an operand whose
+// cp.async two chunks ahead, in the order memory has them: an operand whose
 // inner index is contiguous (W, the input, T, the transposed dense leaves) as
 // rows of 16 inner indices, their eight 16-byte units exchanged between halves
 // on odd rows; the others (U, the dense leaves) as columns of 64 rows with a
@@ -743,8 +746,8 @@ wide_tf32_kernel(const JobExec* __restrict__ jobs, int njobs, const JobExec job0
 // addresses.  A warp whose rows or columns all lie beyond the tile does not
 // multiply; testing that per 8 x 8 block cost more than the blocks (128
 // columns of the 200 x 184 operator: 5 %).  Measured, 64 columns of the 128 x
-// 128 operator (rank 16): 392 -> 283 us for both phases, 16 TF/s of 37; 5
-// columns of the 117 x 101 one, transposed: 147 -> 82 us.
+// 128 operator (rank 16): 392 -> 227 us for both phases, 19 TF/s of 37; 5
+// columns of the 117 x 101 one, transposed: 147 -> 74 us.
 // ---------------------------------------------------------------------------
 template <int NT>
 struct Tile64 {
@@ -752,9 +755,9 @@ struct Tile64 {
     static constexpr int MB = 8 / WM, NB = NT / (8 * WN);      // 8 x 8 blocks of a warp
     static constexpr int STAGES = 3;
     // CTAs an SM: fewer for the wide tiles, whose accumulators and addresses
-    // otherwise spill (64 columns: 3 CTAs 283 us, 4 CTAs 300 us, 4 stages 290
-    // us for the 128 x 128 operator; 8 columns: 6 CTAs 82 us, 5 CTAs 88 us for
-    // 5 columns of the 117 x 101 one)
+    // otherwise spill (when 64 columns of the 128 x 128 operator took 283 us:
+    // 4 CTAs 300 us, 4 stages 290 us; when 5 columns of the 117 x 101 one took
+    // 82 us: 5 CTAs 88 us)
     static constexpr int CTAS = NT == 64 ? 3 : NT == 32 ? 4 : 6;
     static constexpr int ASZ = KC * 66;                        // doubles of an A stage
     static constexpr int BSZ = NT * KC;
@@ -1684,9 +1687,9 @@ void run_jobs_direct(Context& ctx, const std::vector<MatJob>& jobs, bool tf32) {
     // one column: 32-row tiles, work split evenly over all resident warps;
     // more: tiles of 64 rows on the tensor cores (FP64 at the narrowest tile
     // that takes the columns; TF32 when asked, from 9 columns on).  Streaming
-    // kernels on the plain FP64 units took 148 us for 5 columns of the 117 x
-    // 101 operator (rank 12), the 8-column tiles take 98; 139 and 71 us for 4
-    // columns of the 128 x 128 one.
+    // kernels on the plain FP64 units took 147 us for 5 columns of the 117 x
+    // 101 operator (rank 12), the 8-column tiles take 74; 139 and 90 us for 4
+    // columns of the 128 x 128 one, 50 and 15 for 16 x 16 points of rank 4.
     const bool wide = kmax > 1;
     tf32 = tf32 && kmax > 8;
     const int nt = kmax <= 8 ? 8 : kmax <= 16 ? 16 : kmax <= 32 ? 32 : 64;   // FP64 tile columns

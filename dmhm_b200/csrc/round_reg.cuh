@@ -23,10 +23,11 @@
 // the columns cut in step 3 (a third of them on average) are never rotated.
 // Bound: the chain of each elimination and rotation step (a reciprocal square
 // root, a broadcast, one barrier: 700 to 900 cycles) times the 16 warps that
-// fit an SM; the FP64 pipe is 14 % busy.  Measured, all roundings of one H*H
-// product (do_round before): 64^2 grid, rank 16, 35,472 roundings 81.1 -> 16.0
-// ms; SchulzInvert there 1106 -> 237 ms in 28 products; complex 24^2, rank 12,
-// 924 -> 221 ms in 36; FP32, 72 x 68 grid, 765 -> 192 ms in 28.
+// fit an SM; the FP64 pipe is 20 % busy on 64 x 64 blocks, 14 % on 256 x 256.
+// Measured, all roundings of one H*H product (do_round before): 64^2 grid, rank
+// 16, 35,472 roundings 81.1 -> 16.0 ms; SchulzInvert there 1106 -> 237 ms in 28
+// products; complex 24^2, rank 12, 924 -> 208 ms in 36; FP32, 72 x 68 grid, 765
+// -> 192 ms in 28.
 #pragma once
 
 #include "fp64_tiles.cuh"
