@@ -41,8 +41,8 @@ REF_DRIVER = os.path.join(ROOT, "oracle", "_ref", "dmhm_ref_driver")
 # workload, each from one ncu capture (dram__bytes_read.sum +
 # dram__bytes_write.sum) of `python -m dmhm_b200.workloads`: FP64 64-column
 # product phases and the one-vector product
-KERNEL_TRAFFIC = {"hmm_row_tiles": (257.1 + 10.4) * 1e6,
-                  "hmm_lowrank_inner": (127.8 + 46.8) * 1e6,
+KERNEL_TRAFFIC = {"hmm_row_tiles": (252.2 + 9.4) * 1e6,
+                  "hmm_lowrank_inner": (125.0 + 38.0) * 1e6,
                   "hmv_blocks": (276.4 + 3.8) * 1e6}
 
 
