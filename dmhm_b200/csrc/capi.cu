@@ -87,10 +87,11 @@ void Context::collect() {
     pending.clear();
 }
 
-void Context::fork(int n) {
+void Context::fork(int mask) {
     if (!side_fork) HMB_CUDA(cudaEventCreateWithFlags(&side_fork, cudaEventDisableTiming));
     HMB_CUDA(cudaEventRecord(side_fork, stream));
-    for (int i = 0; i < n; ++i) {
+    for (int i = 0; i < kSideStreams; ++i) {
+        if (!(mask >> i & 1)) continue;
         if (!side[i]) {
             int least = 0, greatest = 0, base = 0;
             HMB_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
@@ -103,17 +104,18 @@ void Context::fork(int n) {
     }
 }
 
-void Context::join(int n) {
-    for (int i = 0; i < n; ++i) {
+void Context::join(int mask) {
+    for (int i = 0; i < kSideStreams; ++i) {
+        if (!(mask >> i & 1)) continue;
         HMB_CUDA(cudaEventRecord(side_done[i], side[i]));
         HMB_CUDA(cudaStreamWaitEvent(stream, side_done[i], 0));
     }
 }
 
-void Context::drain(int n) noexcept {
-    for (int i = 0; i < n; ++i)
-        if (cudaEventRecord(side_done[i], side[i]) != cudaSuccess ||
-            cudaStreamWaitEvent(stream, side_done[i], 0) != cudaSuccess) {
+void Context::drain(int mask) noexcept {
+    for (int i = 0; i < kSideStreams; ++i)
+        if ((mask >> i & 1) && (cudaEventRecord(side_done[i], side[i]) != cudaSuccess ||
+                                cudaStreamWaitEvent(stream, side_done[i], 0) != cudaSuccess)) {
             cudaGetLastError();   // (the error that ended the scope is reported)
             cudaStreamSynchronize(side[i]);
         }

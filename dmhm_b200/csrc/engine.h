@@ -97,19 +97,20 @@ struct Context {
     double* pinned_scalar();
     double* pinned = nullptr;
     // Side streams for launches that are independent of one another: fork()
-    // makes `n` of them wait for the work queued on `stream` so far, join()
-    // makes `stream` wait for theirs, so that everything queued on `stream`
-    // afterwards (frees included) follows it; drain() does that without
-    // throwing, waiting on the host where it must.  Used through ForkScope
-    // (fork_scope.h).  Made on first use, each of a higher priority than the
-    // next and all of a higher one than `stream`, so that the CTAs of launches
-    // that become ready together start in the order side[0], side[1], `stream`.
-    static constexpr int kSideStreams = 2;
+    // makes those of a mask (bit i: side[i]) wait for the work queued on
+    // `stream` so far, join() makes `stream` wait for theirs, so that
+    // everything queued on `stream` afterwards (frees included) follows it;
+    // drain() does that without throwing, waiting on the host where it must.
+    // Used through ForkScope (fork_scope.h).  Made on first use, each of a
+    // higher priority than the next and all of a higher one than `stream`, so
+    // that the CTAs of launches that become ready together start in the order
+    // of their streams.
+    static constexpr int kSideStreams = 3;
     cudaStream_t side[kSideStreams] = {};
     cudaEvent_t side_fork = nullptr, side_done[kSideStreams] = {};
-    void fork(int n);
-    void join(int n);
-    void drain(int n) noexcept;
+    void fork(int mask);
+    void join(int mask);
+    void drain(int mask) noexcept;
     void release_side();
     // Device word set by kernels whose bounded waits gave up (zero = fine);
     // read and cleared by check_numerical().

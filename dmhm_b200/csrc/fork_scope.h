@@ -5,27 +5,27 @@
 
 namespace hmb {
 
-// Ctx: fork(n) and join(n) may throw; drain(n) orders (or waits) without.
+// Ctx: fork(mask) and join(mask) may throw; drain(mask) orders (or waits) without.
 template <typename Ctx>
 class ForkScope {
   public:
-    // n side streams (0: nothing to do)
-    ForkScope(Ctx& ctx, int n) : ctx_(ctx), n_(n) {
-        if (n_ > 0) ctx_.fork(n_);
+    // the side streams of a mask (0: nothing to do)
+    ForkScope(Ctx& ctx, int mask) : ctx_(ctx), mask_(mask) {
+        if (mask_ != 0) ctx_.fork(mask_);
     }
     ForkScope(const ForkScope&) = delete;
     ForkScope& operator=(const ForkScope&) = delete;
     void join() {
-        if (n_ > 0) ctx_.join(n_);
-        n_ = 0;
+        if (mask_ != 0) ctx_.join(mask_);
+        mask_ = 0;
     }
     ~ForkScope() {
-        if (n_ > 0) ctx_.drain(n_);
+        if (mask_ != 0) ctx_.drain(mask_);
     }
 
   private:
     Ctx& ctx_;
-    int n_;
+    int mask_;
 };
 
 }  // namespace hmb

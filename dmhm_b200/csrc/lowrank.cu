@@ -754,13 +754,16 @@ void launch_round_reg(const RoundList& L, const int* workers, const RoundList::G
 }
 
 // The groups of a list are independent (each worker writes its own block)
-// and each leaves SMs idle at its end, so they run at the same time, by the
-// priorities of the side streams the general kernel first (its CTAs are the
-// longest), then the 4-warp form, whose CTAs fit beside the others', then the
-// 8-warp one.  Streams of one priority start in an order that changes with the
-// build and with the streams made before: mixed SchulzInvert 72 x 68 took 330
-// ms or, when the general kernel came last and ran on nearly alone, 378; with
-// the 8-warp form second 330 or 353 (64 x 64 product 19.3 ms), so 328 (18.6).
+// and each leaves SMs idle at its end, so they run at the same time, in the
+// order of the side streams' priorities: the general kernel first (its CTAs are
+// the longest), then the 4-warp form, whose CTAs fit beside the others', then
+// the 8-warp one.  All of them wait for the same event; a kernel on the
+// context's own stream starts before or after those that wait, as the build and
+// the streams made before have it (mixed SchulzInvert 72 x 68: 330 ms or, when
+// the general kernel came last and ran on nearly alone, 378; 326 this way;
+// SchulzInvert of 49 x 46 points, 4-warp form ahead of the general kernel 500
+// ms, this way 465; with the 8-warp form second 353 and 64 x 64 product 19.3
+// ms, this way 18.5).
 template <typename R>
 void launch_round_typed(Context& ctx, const RoundList& L, const RelocBases& bases,
                         const char* name) {
@@ -779,24 +782,19 @@ void launch_round_typed(Context& ctx, const RoundList& L, const RelocBases& base
     }
     LaunchScope ls(ctx, name);
     g_launches.fetch_add(parts - 1, std::memory_order_relaxed);
-    ForkScope<Context> fork(ctx, parts - 1);
-    int next = 0;   // the last part stays on the context's stream
-    auto stream = [&]() {
-        const int i = next++;
-        return i < parts - 1 ? ctx.side[i] : ctx.stream;
-    };
+    const int mask = (sch.nw_general > 0 ? 1 : 0) | (sch.groups[1].count > 0 ? 2 : 0) |
+                     (sch.groups[0].count > 0 ? 4 : 0);
+    ForkScope<Context> fork(ctx, parts > 1 ? mask : 0);
+    auto stream = [&](int i) { return parts > 1 ? ctx.side[i] : ctx.stream; };
     if (sch.nw_general > 0) {
-        round_worker_kernel<R><<<(unsigned)sch.nw_general, kT, sch.smem * sizeof(R), stream()>>>(
+        round_worker_kernel<R><<<(unsigned)sch.nw_general, kT, sch.smem * sizeof(R), stream(0)>>>(
             L.ops.get(), L.index.get(), workers, sch.smem, bases, numflag);
         HMB_CHECK_LAUNCH();
     }
-    for (int i = 1; i >= 0; --i) {   // 4 warps, then 8
-        const RoundList::Group& g = sch.groups[i];
-        if (g.count == 0) continue;
-        const cudaStream_t st = stream();
-        if (g.warps == 4) launch_round_reg<R, 4>(L, workers, g, bases, numflag, st);
-        else launch_round_reg<R, 8>(L, workers, g, bases, numflag, st);
-    }
+    if (sch.groups[1].count > 0)
+        launch_round_reg<R, 4>(L, workers, sch.groups[1], bases, numflag, stream(1));
+    if (sch.groups[0].count > 0)
+        launch_round_reg<R, 8>(L, workers, sch.groups[0], bases, numflag, stream(2));
     fork.join();
 }
 
