@@ -31,6 +31,7 @@
 #pragma once
 
 #include "fp64_tiles.cuh"
+#include "reciprocal.cuh"
 #include "round_sizing.h"
 
 namespace hmb {
@@ -211,10 +212,6 @@ __device__ __forceinline__ void sum_slabs(const Cta<R, NW>& C, int buf, R (&s)[C
     }
 }
 
-// (FP64: a call-free form of 1 / x; every step waits for it)
-__device__ __forceinline__ double reciprocal(double x) { return __drcp_rn(x); }
-__device__ __forceinline__ float reciprocal(float x) { return 1.0f / x; }
-
 // One elimination step: the reflector of column p on row j (the first row of
 // the owning warp's slab), applied to all columns.  On return t holds row j of
 // R for this lane's columns, the owner's slab has moved up by one row and us
@@ -264,8 +261,8 @@ __device__ __forceinline__ Reflector<R> eliminate(const Cta<R, NW> C, R (&a)[CPL
         // beta = -sign(alpha) h, h = ||x||; u0 = alpha - beta; tau1 = -u0 / beta
         const R h2 = r_fma(alpha, alpha, sigma), rs = r_rsqrt(h2), h = h2 * rs;
         H.u0 = alpha + r_copysign(h, alpha);
-        scal = reciprocal(H.u0);
         tau1 = r_fma(r_abs(alpha), rs, R(1));
+        scal = reciprocal(H.u0);
         H.tau = tau1 * scal * scal;
     }
 #pragma unroll
